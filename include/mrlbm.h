@@ -161,6 +161,11 @@ int mrlbm_set_inlet_profile(mrlbm_handle* h, const double* u_in);
  * the steps post_process and statsbegin <= iter <= statsend select (2d_mrlbm.f90:461-502).
  * With flags & MRLBM_STEP_MACRO the last step also stores its post-boundary-condition
  * macroscopic fields for mrlbm_get_macro. */
+/* On large lattices a call takes its steps two at a time (each pair reads and writes the
+ * populations once; the same bits as two single steps), a last odd step and a step with macroscopic output
+ * alone.  Pairs need a third population level on the device; without the memory for it, and on
+ * x-slabs, steps are single.  The rule is by size and precision, mrlbm_autotune replaces it by a
+ * measurement, and MRLBM_PAIRS=0 or 1 in the environment at creation replaces both. */
 #define MRLBM_STEP_MACRO   1
 int mrlbm_step(mrlbm_handle* h, int32_t nsteps, int32_t flags);
 
@@ -252,8 +257,9 @@ int mrlbm_get_tile_config(const mrlbm_handle* h, int32_t* cfg);
  * warm-up step each), keep the fastest, and restore the populations, the iteration counter
  * and the force history, so a simulation is unaffected.  Trial steps record no surface
  * pressure; with a field-statistics window they accumulate like the run will (so the choice
- * fits it) into sums that are saved beforehand and put back.  Returns the chosen shape and its
- * time per step in milliseconds. */
+ * fits it) into sums that are saved beforehand and put back.  With the fastest shape it then
+ * times the steps in pairs (mrlbm_step) and keeps whichever is faster.  Returns the chosen shape
+ * (of single steps) and the time per step in milliseconds. */
 int mrlbm_autotune(mrlbm_handle* h, int32_t trial_steps, int32_t* best_cfg, double* best_ms);
 
 /* Field statistics (no counterpart in the reference, whose 2d_statistics post-processes

@@ -26,6 +26,8 @@ NVCC_COMMON = ARCH + ["-lineinfo", "-O3", "-std=c++17", "--expt-relaxed-constexp
 CU_UNITS = {
     "step_f64.cu": ["-fmad=false"],
     "step_f32.cu": [],
+    "pair_f64.cu": ["-fmad=false"],
+    "pair_f32.cu": [],
     "adjoint.cu": [],
     "noalloc.cu": [],
     "state_io.cu": [],

@@ -20,6 +20,7 @@
 #include "noalloc.h"
 #include "state_io.h"
 #include "surface.h"
+#include "step_pair.h"
 #include "step_params.h"
 
 using namespace mrlbm;
@@ -44,6 +45,11 @@ struct mrlbm_handle {
     size_t elem = 8;
     void* buf[2] = {nullptr, nullptr};
     int cur = 0;
+    // steps taken in pairs (step_pair.cuh): the buffer of the intermediate level's band
+    bool pairs = false, pairs_fixed = false;  // fixed: by the environment, not by rule or autotuner
+    void* mid = nullptr;
+    PairPlan plan{};
+    CUtensorMap tmap_pair[2];                 // 3-D maps (columns, rows, planes) of both time levels
     void* d_bgeo = nullptr;
     int* d_bint = nullptr;
     int* d_boxmap = nullptr;
@@ -215,6 +221,7 @@ int upload_state(mrlbm_handle* h, const double* f) {
         CK(cudaMemcpyAsync(h->d_ovr, h->ovr.data(), h->ovr.size() * sizeof(OvrEntry), cudaMemcpyHostToDevice,
                            h->stream));
     }
+    if (h->mid) CK(launch_copy_ring(h->precision, h->buf[0], h->mid, h->L, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     h->ovr_live = !h->ovr.empty();
     return MRLBM_OK;
@@ -489,10 +496,138 @@ int launch_one(mrlbm_handle* h, bool stats, bool plot, bool macro) {
     return MRLBM_OK;
 }
 
+// Whether the handle's lattice can be stepped in pairs at all.
+bool pairs_possible(const mrlbm_handle* h) {
+    return !h->halo_l && !h->halo_r && h->L.nx >= PAIR_MIN_NX && h->L.ny >= PAIR_MIN_NY;
+}
+
+// Whether pairs are taken from the start (the autotuner measures instead).  Below about a million FP64 or
+// two million FP32 nodes a step is bound by the wall nodes' latency and the launches, of which a pair
+// has as many.  Single steps and pairs, us per step: 1003 x 251 8.5 and 10.5 (FP64), 8.0 and 11.4 (FP32);
+// 2048 x 512 25.9 and 20.3, 11.4 and 13.2; 2900 x 725 50.8 and 35.4, 27.3 and 21.0; 4099 x 1023 97 and 63, 52 and 37.
+bool pairs_pay(const mrlbm_handle* h) {
+    const int64_t nodes = (int64_t)h->L.nx * h->L.ny;
+    return std::min(h->L.nx, h->L.ny) >= 64 && nodes >= (h->precision == MRLBM_FP64 ? 700000 : 1500000);
+}
+
+// Nodes the two-step tiles leave out and the band of the intermediate level (PairPlan).
+void make_pair_plan(mrlbm_handle* h) {
+    const Geometry& g = h->geo;
+    PairPlan& q = h->plan;
+    q.core = q.halo = PairRect{1, 0, 1, 0};
+    if (g.box_w > 0) {
+        q.core = PairRect{g.box_x0 - 1, g.box_x0 + g.box_w, g.box_y0 - 1, g.box_y0 + g.box_h};
+        q.halo = PairRect{q.core.x0 - 1, q.core.x1 + 1, q.core.y0 - 1, q.core.y1 + 1};
+        for (int l = 0; l < g.nb; ++l)
+            for (int m = 0; m < 8; ++m) {
+                const int i = g.tint[(size_t)(I_SI + m) * g.nb + l], j = g.tint[(size_t)(I_SJ + m) * g.nb + l];
+                q.halo.x0 = std::min(q.halo.x0, i - 1);
+                q.halo.x1 = std::max(q.halo.x1, i + 1);
+                q.halo.y0 = std::min(q.halo.y0, j - 1);
+                q.halo.y1 = std::max(q.halo.y1, j + 1);
+            }
+    }
+    q.chunks = pair_chunks(h->L.nx, h->L.ny, h->elem == 8 ? PAIR_STRIPS64 : PAIR_STRIPS32, PAIR_MINB * h->num_sms);
+}
+
+// Take steps in pairs from now on: the band buffer, with the ghost ring every level carries.
+// False (and single steps as before) when there is no memory for it.
+bool enable_pairs(mrlbm_handle* h) {
+    if (!pairs_possible(h)) return false;
+    if (!h->mid) {
+        auto enc = tensor_map_encoder();
+        if (!enc) return false;
+        for (int b = 0; b < 2; ++b) {
+            cuuint64_t dims[3] = {(cuuint64_t)h->L.pitch, (cuuint64_t)h->L.ny + 2, (cuuint64_t)Q};
+            cuuint64_t strides[2] = {(cuuint64_t)h->L.pitch * h->elem, (cuuint64_t)h->L.plane * h->elem};
+            cuuint32_t box[3] = {(cuuint32_t)pair_box_cols(h->elem == 8 ? PAIR_STRIPS64 : PAIR_STRIPS32), 1, (cuuint32_t)Q}, estr[3] = {1, 1, 1};
+            if (enc(&h->tmap_pair[b], h->elem == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3,
+                    h->buf[b], dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+                return false;
+        }
+        if (cudaMalloc(&h->mid, (size_t)h->L.total() * h->elem) != cudaSuccess) {
+            cudaGetLastError();
+            h->mid = nullptr;
+            return false;
+        }
+        if (launch_copy_ring(h->precision, h->buf[h->cur], h->mid, h->L, h->stream) != cudaSuccess) return false;
+        make_pair_plan(h);
+    }
+    h->pairs = true;
+    return true;
+}
+
+void disable_pairs(mrlbm_handle* h) {
+    h->pairs = false;
+    if (h->mid) cudaFree(h->mid);
+    h->mid = nullptr;
+}
+
+bool stats_at(const mrlbm_handle* h, int iter) {
+    return h->cfg.post_process && iter >= h->cfg.statsbegin && iter <= h->cfg.statsend;
+}
+bool plot_at(const mrlbm_handle* h, int iter) {
+    const mrlbm_config& c = h->cfg;
+    return c.post_process && c.iplot > 0 && iter % c.iplot == 0 && (c.channel_with_cylinder || c.channel_with_square);
+}
+bool fields_at(const mrlbm_handle* h, int iter) { return h->d_fstat && iter >= h->fstat_begin && iter <= h->fstat_end; }
+
+// Whether the next two steps can be one pair: no loaded-state overrides, no surface record, both
+// steps or neither inside the field-statistics window, room for both records in the ring.
+bool pair_ok(const mrlbm_handle* h) {
+    const int a = h->iter + 1, b = h->iter + 2;
+    return h->pairs && !h->ovr_live && h->ring_n + 2 <= RING_CAP && fields_at(h, a) == fields_at(h, b) &&
+           !(h->surf_on && (stats_at(h, a) || stats_at(h, b)));
+}
+
+template <class T>
+int launch_pair_t(mrlbm_handle* h) {
+    StepParams<T> p[2];
+    for (int q = 0; q < 2; ++q) {
+        const int iter = h->iter + 1 + q;
+        const bool stats = stats_at(h, iter);
+        p[q] = StepParams<T>{};
+        fill_common(h, p[q]);
+        set_deferred(h, p[q]);
+        p[q].src = (const T*)(q == 0 ? h->buf[h->cur] : h->mid);
+        p[q].dst = (T*)(q == 0 ? h->mid : h->buf[1 - h->cur]);
+        p[q].u_in = h->has_uin ? (const T*)h->d_uin : nullptr;
+        p[q].body = h->has_body ? (const T*)h->d_body : nullptr;
+        p[q].zero_solid_u = plot_at(h, iter);
+        p[q].do_stats = stats;
+        p[q].rec = stats ? h->d_ring + (size_t)h->ring_n * REC_WORDS : nullptr;
+        p[q].iter = iter;
+        if (q == 0) p[q].tmap = h->tmap_pair[h->cur];
+        p[q].fstat = fields_at(h, iter) ? h->d_fstat : nullptr;
+        h->pend.on = false;
+        if (stats) {
+            h->pend = mrlbm_handle::Pending{true, h->pslot, h->ring_n, iter};
+            h->pslot ^= 1;
+            ++h->ring_n;
+        }
+        if (p[q].fstat) ++h->fstat_n;
+    }
+    if constexpr (sizeof(T) == 8) return launch_pair_f64(p[0], p[1], h->plan, h->cur != 0, h->stream);
+    else return launch_pair_f32(p[0], p[1], h->plan, h->cur != 0, h->stream);
+}
+
+int launch_two(mrlbm_handle* h) {
+    const int rc = h->precision == MRLBM_FP64 ? launch_pair_t<double>(h) : launch_pair_t<float>(h);
+    if (rc != 0) {
+        h->err = std::string("kernel launch failed: ") + cudaGetErrorString(cudaGetLastError());
+        return MRLBM_ECUDA;
+    }
+    h->launches += PAIR_LAUNCHES;
+    h->iter += 2;
+    h->cur ^= 1;
+    return MRLBM_OK;
+}
+
 void free_all(mrlbm_handle* h) {
     if (h->host_only) return;
     cudaSetDevice(h->device);
-    for (void* p : {h->buf[0], h->buf[1], h->d_bgeo, (void*)h->d_bint, (void*)h->d_boxmap, (void*)h->d_partials,
+    for (void* p : {h->buf[0], h->buf[1], h->mid, h->d_bgeo, (void*)h->d_bint, (void*)h->d_boxmap, (void*)h->d_partials,
                     (void*)h->d_counter, (void*)h->d_ring, (void*)h->d_err, (void*)h->d_macro, (void*)h->d_uin, h->d_body, (void*)h->d_ovr, h->adj_ws, (void*)h->d_fstage,
                     (void*)h->d_tile_ctr, (void*)h->d_fstat, (void*)h->d_fstat_out, (void*)h->d_quad, (void*)h->d_W,
                     (void*)h->d_sumw, (void*)h->d_sring, (void*)h->d_pring, (void*)h->d_sidx})
@@ -712,6 +847,9 @@ static int create_impl(const mrlbm_config* cfg, int precision, int device, int s
     // the main loop runs iter = restart_step+1, ... with restart_step initialised to 1
     // (2d_mrlbm.f90:7, 229): a fresh run's first step is iter 2
     h->iter = 1;
+    const char* pv = std::getenv("MRLBM_PAIRS");
+    h->pairs_fixed = pv != nullptr;
+    if (pv ? std::atoi(pv) != 0 : pairs_pay(h)) enable_pairs(h);
     *out = h;
     return MRLBM_OK;
 }
@@ -1169,19 +1307,24 @@ int mrlbm_step(mrlbm_handle* h, int32_t nsteps, int32_t flags) {
     if (!h || nsteps < 0) return MRLBM_EINVAL;
     if (h->host_only) return fail(h, MRLBM_ENODEVICE, "host-only handle (created with device -1)");
     CK(cudaSetDevice(h->device));
-    const mrlbm_config& c = h->cfg;
     if ((flags & MRLBM_STEP_MACRO) && !h->d_macro)
         CK(cudaMalloc((void**)&h->d_macro, (size_t)6 * h->L.nx * h->L.ny * sizeof(double)));
-    for (int s = 0; s < nsteps; ++s) {
-        h->iter += 1;
-        const bool stats = c.post_process && h->iter >= c.statsbegin && h->iter <= c.statsend;
-        const bool plot = c.post_process && c.iplot > 0 && h->iter % c.iplot == 0 &&
-                          (c.channel_with_cylinder || c.channel_with_square);
-        const bool macro = (flags & MRLBM_STEP_MACRO) && s == nsteps - 1;
-        int rc = launch_one(h, stats, plot, macro);
-        if (rc != MRLBM_OK) {
-            if (rc == MRLBM_EUNSUPPORTED) h->iter -= 1;      // nothing was launched
-            return rc;
+    for (int s = 0; s < nsteps;) {
+        int rc;
+        // a step with macroscopic output is taken alone
+        if (nsteps - s >= ((flags & MRLBM_STEP_MACRO) ? 3 : 2) && pair_ok(h)) {
+            rc = launch_two(h);
+            if (rc != MRLBM_OK) return rc;
+            s += 2;
+        } else {
+            h->iter += 1;
+            const bool macro = (flags & MRLBM_STEP_MACRO) && s == nsteps - 1;
+            rc = launch_one(h, stats_at(h, h->iter), plot_at(h, h->iter), macro);
+            if (rc != MRLBM_OK) {
+                if (rc == MRLBM_EUNSUPPORTED) h->iter -= 1;      // nothing was launched
+                return rc;
+            }
+            ++s;
         }
         if (h->ring_n == RING_CAP) {
             rc = drain_ring(h);
@@ -1368,9 +1511,20 @@ int mrlbm_autotune(mrlbm_handle* h, int32_t trial_steps, int32_t* best_cfg, doub
     int best = cfg0;
     float best_t = 1e30f;
     int rc = MRLBM_OK;
-    for (int c = 0; c < N_ALL_CFGS && rc == MRLBM_OK; ++c) {
-        h->tile_cfg = c;
-        rc = mrlbm_step(h, 1, 0);                       // warm-up (and instruction cache)
+    // every shape by single steps, then (index N_ALL_CFGS) the best of them with its steps in pairs
+    const bool pairs0 = h->pairs;
+    const int last = h->pairs_fixed || std::min(h->L.nx, h->L.ny) < 64 ? N_ALL_CFGS : N_ALL_CFGS + 1;
+    bool pairs_best = false;
+    for (int c = 0; c < last && rc == MRLBM_OK; ++c) {
+        const bool paired = c == N_ALL_CFGS;
+        h->pairs = h->pairs_fixed ? pairs0 : false;
+        if (paired) {
+            if (best_t >= 1e30f || !enable_pairs(h)) break;
+            h->tile_cfg = best;
+        } else {
+            h->tile_cfg = c;
+        }
+        rc = mrlbm_step(h, paired ? 2 : 1, 0);          // warm-up (and instruction cache)
         if (rc == MRLBM_EUNSUPPORTED) {                 // shape does not fit: nothing ran
             rc = MRLBM_OK;
             h->iter = iter0;
@@ -1383,7 +1537,11 @@ int mrlbm_autotune(mrlbm_handle* h, int32_t trial_steps, int32_t* best_cfg, doub
         if (rc != MRLBM_OK || cudaEventSynchronize(e1) != cudaSuccess) { rc = rc ? rc : MRLBM_ECUDA; break; }
         float ms = 0.f;
         cudaEventElapsedTime(&ms, e0, e1);
-        if (ms < best_t) { best_t = ms; best = c; }
+        if (ms < best_t) {
+            best_t = ms;
+            if (paired) pairs_best = true;
+            else best = c;
+        }
         // restore before the next trial so every shape starts from the same state
         for (int b = 0; b < 2; ++b)
             if (cudaMemcpyAsync(h->buf[b], save[b], bytes, cudaMemcpyDeviceToDevice, h->stream) != cudaSuccess)
@@ -1410,9 +1568,13 @@ int mrlbm_autotune(mrlbm_handle* h, int32_t trial_steps, int32_t* best_cfg, doub
     cleanup();
     if (rc != MRLBM_OK) {
         h->tile_cfg = cfg0;
+        h->pairs = pairs0;
         return rc;
     }
     h->tile_cfg = best;
+    if (h->pairs_fixed) h->pairs = pairs0;
+    else if (pairs_best) h->pairs = true;
+    else disable_pairs(h);
     if (best_cfg) *best_cfg = best;
     if (best_ms) *best_ms = best_t / trial_steps;
     return MRLBM_OK;
@@ -2107,6 +2269,7 @@ int mrlbm_batch_create(const mrlbm_config* cfgs, int32_t ncases, int precision, 
             h->own_stream = nullptr;
         }
         h->stream = b->stream;
+        disable_pairs(h);                              // a batch steps its cases one step at a time
     }
     b->stage_bytes = batch_param_bytes(b);
     bool ok = cudaMalloc(&b->d_params, b->stage_bytes) == cudaSuccess &&

@@ -86,6 +86,26 @@ cudaError_t launch_fill_overrides(int precision, const double* f0, OvrEntry* ovr
 }
 
 namespace {
+// Rows 0 and ny + 1 and columns 0 and nx + 1 of the nine planes, one thread per ghost slot.
+template <class T>
+__global__ void copy_ring(const T* __restrict__ src, T* dst, Layout L) {
+    const int per = 2 * (L.nx + 2) + 2 * L.ny, t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (t >= per * Q) return;
+    const int k = t / per, q = t - k * per, row = 2 * (L.nx + 2);
+    const int i = q < row ? q % (L.nx + 2) : ((q - row) & 1) * (L.nx + 1);
+    const int j = q < row ? (q / (L.nx + 2)) * (L.ny + 1) : 1 + (q - row) / 2;
+    dst[L.at(i, j, k)] = src[L.at(i, j, k)];
+}
+}  // namespace
+
+cudaError_t launch_copy_ring(int precision, const void* src, void* dst, const Layout& L, cudaStream_t s) {
+    const unsigned blocks = (unsigned)((Q * (2 * (L.nx + 2) + 2 * L.ny) + 255) / 256);
+    if (precision == 64) copy_ring<double><<<blocks, 256, 0, s>>>((const double*)src, (double*)dst, L);
+    else copy_ring<float><<<blocks, 256, 0, s>>>((const float*)src, (float*)dst, L);
+    return cudaGetLastError();
+}
+
+namespace {
 __global__ void field_stats_finalize(const double* __restrict__ sums, double* __restrict__ out, int64_t N, double n) {
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < N; q += (int64_t)gridDim.x * blockDim.x) {
 #pragma unroll

@@ -23,4 +23,7 @@ cudaError_t launch_fill_overrides(int precision, const double* f0, OvrEntry* ovr
 // fluctuation sqrt(max(<x^2> - <x>^2, 0)) (3 x N).
 cudaError_t launch_field_stats_finalize(const double* sums, double* out, int64_t N, int64_t n, cudaStream_t s);
 
+// The ghost ring (row 0, row ny + 1, column 0, column nx + 1) of one level into another.
+cudaError_t launch_copy_ring(int precision, const void* src, void* dst, const Layout& L, cudaStream_t s);
+
 }  // namespace mrlbm

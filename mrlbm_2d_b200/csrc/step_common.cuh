@@ -123,6 +123,17 @@ __device__ __forceinline__ void fields_load(const StepParams<T>& p, int i, int j
     for (int c = 0; c < 6; ++c) q.v[c] = __ldg(p.fstat + n + c * N);
 }
 
+// The sums after one more step's values, still in registers.
+__device__ __forceinline__ void fields_add(FieldPre& q, double rho, double ux, double uy) {
+    const double pr = __dmul_rn(rho, 1.0 / 3.0);
+    q.v[0] = __dadd_rn(q.v[0], ux);
+    q.v[1] = __dadd_rn(q.v[1], uy);
+    q.v[2] = __dadd_rn(q.v[2], pr);
+    q.v[3] = __dadd_rn(q.v[3], __dmul_rn(ux, ux));
+    q.v[4] = __dadd_rn(q.v[4], __dmul_rn(uy, uy));
+    q.v[5] = __dadd_rn(q.v[5], __dmul_rn(pr, pr));
+}
+
 template <class T>
 __device__ __forceinline__ void fields_store(const StepParams<T>& p, int i, int j, const FieldPre& q, double rho,
                                              double ux, double uy) {

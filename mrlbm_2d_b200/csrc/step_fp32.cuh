@@ -10,6 +10,7 @@
 // w_k + g_k.  Every curved-wall closure of the FP64 step has an FP32 form (rotated strong,
 // weak and rho_eq, unrotated with Cramer's rule, none).
 #pragma once
+#include <type_traits>
 #include "step_common.cuh"
 
 namespace mrlbm {
@@ -30,26 +31,76 @@ __device__ __forceinline__ float rcp_approx(float x) {
     return r;
 }
 
+// The node arithmetic (moments, collide) is written once for single floats and for two nodes at a
+// time (F2: the packed FP32 instructions of sm_100, one instruction slot for two results), with
+// every multiply-add spelled out, so a node rounds the same in every kernel and in either form.
+struct F2 { unsigned long long v; };
+__device__ __forceinline__ F2 f2(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void split(F2 a, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v)); }
+__device__ __forceinline__ F2 add(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 sub(F2 a, F2 b) { F2 r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 mul(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 fma(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 rcp(F2 a) {
+    float x, y;
+    split(a, x, y);
+    return f2(rcp_approx(x), rcp_approx(y));
+}
+// A product that stays one: a packed product may be contracted into a packed sum that follows it, which
+// happens when a kernel takes a node's output straight into the next step's sums.
+__device__ __forceinline__ F2 product(F2 a, F2 b) {
+    float x, y, u, v;
+    split(a, x, y);
+    split(b, u, v);
+    return f2(__fmul_rn(x, u), __fmul_rn(y, v));
+}
+__device__ __forceinline__ float product(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float sub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float rcp(float a) { return rcp_approx(a); }
+template <class S> __device__ __forceinline__ S all(float a);
+template <> __device__ __forceinline__ float all<float>(float a) { return a; }
+template <> __device__ __forceinline__ F2 all<F2>(float a) { return f2(a, a); }
+
+template <class S>
+struct MacS { S drho, rho, ux, uy, mxx, myy, mxy; };
+
 // rho = 1 + sum g + (sum w - 1); u = sum f c / rho; m = sum f H / rho with
 // sum f H_xx = (sum_k w_k H_xx,k) + sum g c_x^2 - sum g / 3.
-__device__ __forceinline__ Mac moments(const P& p, const float g[Q]) {
-    Mac m;
-    const float dg = (((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + (g[6] + g[7]))) + g[8];
-    m.drho = dg + p.dc.eps_mass;
-    m.rho = 1.0f + m.drho;
-    const float inv = rcp_approx(m.rho);
-    const float jx = ((g[1] - g[3]) + (g[5] - g[7])) + (g[8] - g[6]);
-    const float jy = ((g[2] - g[4]) + (g[5] - g[7])) + (g[6] - g[8]);
-    const float d4 = (g[5] + g[6]) + (g[7] + g[8]);
-    const float sxx = (g[1] + g[3]) + d4;
-    const float syy = (g[2] + g[4]) + d4;
-    const float sxy = (g[5] - g[6]) + (g[7] - g[8]);
-    m.ux = jx * inv;
-    m.uy = jy * inv;
-    m.mxx = ((sxx - THIRD * dg) + p.dc.cxx) * inv;
-    m.myy = ((syy - THIRD * dg) + p.dc.cyy) * inv;
-    m.mxy = sxy * inv;
+template <class S>
+__device__ __forceinline__ MacS<S> moments_of(const P& p, const S g[Q]) {
+    MacS<S> m;
+    const S dg = add(add(add(add(g[0], g[1]), add(g[2], g[3])), add(add(g[4], g[5]), add(g[6], g[7]))), g[8]);
+    m.drho = add(dg, all<S>(p.dc.eps_mass));
+    m.rho = add(all<S>(1.0f), m.drho);
+    const S inv = rcp(m.rho);
+    const S jx = add(add(sub(g[1], g[3]), sub(g[5], g[7])), sub(g[8], g[6]));
+    const S jy = add(add(sub(g[2], g[4]), sub(g[5], g[7])), sub(g[6], g[8]));
+    const S d4 = add(add(g[5], g[6]), add(g[7], g[8]));
+    const S sxx = add(add(g[1], g[3]), d4);
+    const S syy = add(add(g[2], g[4]), d4);
+    const S sxy = add(sub(g[5], g[6]), sub(g[7], g[8]));
+    m.ux = mul(jx, inv);
+    m.uy = mul(jy, inv);
+    m.mxx = mul(add(fma(all<S>(-THIRD), dg, sxx), all<S>(p.dc.cxx)), inv);
+    m.myy = mul(add(fma(all<S>(-THIRD), dg, syy), all<S>(p.dc.cyy)), inv);
+    m.mxy = mul(sxy, inv);
     return m;
+}
+
+__device__ __forceinline__ Mac moments(const P& p, const float g[Q]) {
+    const MacS<float> m = moments_of<float>(p, g);
+    return Mac{m.drho, m.rho, m.ux, m.uy, m.mxx, m.myy, m.mxy};
 }
 
 __device__ __forceinline__ float hxx_of(int k, float hm, float hp) { return ex(k) != 0 ? hp : hm; }
@@ -148,30 +199,40 @@ __device__ __forceinline__ void edge_node(const P& p, int i, int j, const float 
 
 // Moment-space collision and Hermite reconstruction (2d_mrlbm.f90:407-457) on deviations:
 // g_out_k = w_k (drho + rho a_k), a_k = 3 c_k.u + 4.5 m_xx H_xx,k + 4.5 m_yy H_yy,k + 9 m_xy H_xy,k.
-__device__ __forceinline__ void collide(const P& p, const Mac& m, float go[Q]) {
-    const float om = p.omega, om1 = p.omega1;
-    float mxx = om1 * m.mxx + om * m.ux * m.ux;
-    float myy = om1 * m.myy + om * m.uy * m.uy;
-    const float mxy = om1 * m.mxy + om * m.ux * m.uy;
-    if (p.incomp_bulk) {
-        const float t = 0.5f * (mxx + myy - m.ux * m.ux - m.uy * m.uy);
-        mxx -= t;
-        myy -= t;
+template <class S>
+__device__ __forceinline__ void collide_of(const P& p, const MacS<S>& m, S go[Q]) {
+    const S om = all<S>(p.omega), om1 = all<S>(p.omega1);
+    const S ox = mul(om, m.ux), oy = mul(om, m.uy);
+    S mxx = fma(om1, m.mxx, mul(ox, m.ux));
+    S myy = fma(om1, m.myy, mul(oy, m.uy));
+    const S mxy = fma(om1, m.mxy, mul(ox, m.uy));
+    if (p.incomp_bulk) {                           // m - t I, t = (tr m - |u|^2) / 2
+        const S minus = all<S>(-1.0f);
+        const S t = mul(all<S>(0.5f), fma(mul(minus, m.uy), m.uy, fma(mul(minus, m.ux), m.ux, add(mxx, myy))));
+        mxx = sub(mxx, t);
+        myy = sub(myy, t);
     }
-    const float A = 4.5f * mxx, B = 4.5f * myy, C = 9.0f * mxy;
-    const float hm = p.hm, hp = p.hp;
-    const float b0 = (A + B) * hm, bx = A * hp + B * hm, by = A * hm + B * hp, bd = (A + B) * hp;
-    const float tx = 3.0f * m.ux, ty = 3.0f * m.uy, tp = 3.0f * (m.ux + m.uy), tm = 3.0f * (m.ux - m.uy);
-    const float r = m.rho, d = m.drho;
-    go[0] = p.w[0] * (d + r * b0);
-    go[1] = p.w[1] * (d + r * (bx + tx));
-    go[2] = p.w[1] * (d + r * (by + ty));
-    go[3] = p.w[1] * (d + r * (bx - tx));
-    go[4] = p.w[1] * (d + r * (by - ty));
-    go[5] = p.w[5] * (d + r * ((bd + C) + tp));
-    go[6] = p.w[5] * (d + r * ((bd - C) - tm));
-    go[7] = p.w[5] * (d + r * ((bd + C) - tp));
-    go[8] = p.w[5] * (d + r * ((bd - C) + tm));
+    const S A = mul(all<S>(4.5f), mxx), B = mul(all<S>(4.5f), myy);
+    const S hm = all<S>(p.hm), hp = all<S>(p.hp), AB = add(A, B);
+    const S b0 = mul(AB, hm), bd = mul(AB, hp);
+    const S bx = fma(B, hm, mul(A, hp)), by = fma(A, hm, mul(B, hp));
+    const S bp = fma(all<S>(9.0f), mxy, bd), bm = fma(all<S>(-9.0f), mxy, bd);
+    const S three = all<S>(3.0f), less = all<S>(-3.0f), up = add(m.ux, m.uy), um = sub(m.ux, m.uy);
+    const S r = m.rho, d = m.drho, w0 = all<S>(p.w[0]), w1 = all<S>(p.w[1]), w5 = all<S>(p.w[5]);
+    // 0, 2 and 4 move to no other column: the next step of the same lane may take them as they are
+    go[0] = product(w0, fma(r, b0, d));
+    go[1] = mul(w1, fma(r, fma(three, m.ux, bx), d));
+    go[2] = product(w1, fma(r, fma(three, m.uy, by), d));
+    go[3] = mul(w1, fma(r, fma(less, m.ux, bx), d));
+    go[4] = product(w1, fma(r, fma(less, m.uy, by), d));
+    go[5] = mul(w5, fma(r, fma(three, up, bp), d));
+    go[6] = mul(w5, fma(r, fma(less, um, bm), d));
+    go[7] = mul(w5, fma(r, fma(less, up, bp), d));
+    go[8] = mul(w5, fma(r, fma(three, um, bm), d));
+}
+
+__device__ __forceinline__ void collide(const P& p, const Mac& m, float go[Q]) {
+    collide_of<float>(p, MacS<float>{m.drho, m.rho, m.ux, m.uy, m.mxx, m.myy, m.mxy}, go);
 }
 
 // Velocity and rotated second moments of one bilinear stencil node (2d_mrlbm.f90:842-867).
@@ -433,6 +494,35 @@ struct PhysicsT {
     static __device__ __forceinline__ void finish(const P& p, int i, int j, int cls, const T g[Q]) {
         fp32::finish<FULL>(p, i, j, cls, g);
     }
+    // Plain interior nodes (no wall, edge or solid handling), n at a time: populations f[k][.] in,
+    // g[k][.] out, the macroscopic values returned in m.  Two nodes go through the packed form.
+    using M = Mac;
+    template <int N>
+    static __device__ __forceinline__ void plain(const P& p, const T (&f)[Q][N], T (&g)[Q][N], M (&m)[N]) {
+        static_assert(N == 1 || N == 2, "one or two nodes");
+        using S = typename std::conditional<N == 1, float, F2>::type;
+        S a[Q], o[Q];
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+            if constexpr (N == 1) a[k] = f[k][0];
+            else a[k] = f2(f[k][0], f[k][1]);
+        }
+        const MacS<S> q = moments_of<S>(p, a);
+        collide_of<S>(p, q, o);
+        if constexpr (N == 1) {
+            m[0] = Mac{q.drho, q.rho, q.ux, q.uy, q.mxx, q.myy, q.mxy};
+#pragma unroll
+            for (int k = 0; k < Q; ++k) g[k][0] = o[k];
+        } else {
+            split(q.drho, m[0].drho, m[1].drho);
+            split(q.rho, m[0].rho, m[1].rho);
+            split(q.ux, m[0].ux, m[1].ux);
+            split(q.uy, m[0].uy, m[1].uy);
+#pragma unroll
+            for (int k = 0; k < Q; ++k) split(o[k], g[k][0], g[k][1]);
+        }
+    }
+    static __device__ __forceinline__ double rho_of(const M& m) { return 1.0 + (double)m.drho; }
     static __device__ __forceinline__ double edge_bulk_node(const P& p, int i, int j, int cls) {
         return fp32::edge_bulk_node<FULL>(p, i, j, cls);
     }

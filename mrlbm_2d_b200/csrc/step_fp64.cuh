@@ -464,6 +464,23 @@ struct PhysicsT {
     static __device__ __forceinline__ void finish(const P& p, int i, int j, int cls, const T f[Q]) {
         fp64::finish<FULL>(p, i, j, cls, f);
     }
+    // Plain interior nodes (no wall, edge or solid handling), n at a time: populations f[k][.] in,
+    // g[k][.] out, the macroscopic values returned in m.
+    using M = Mac;
+    template <int N>
+    static __device__ __forceinline__ void plain(const P& p, const T (&f)[Q][N], T (&g)[Q][N], M (&m)[N]) {
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            T a[Q], o[Q];
+#pragma unroll
+            for (int k = 0; k < Q; ++k) a[k] = f[k][n];
+            m[n] = moments(a, p.hm, p.hp);
+            collide(p, m[n], o);
+#pragma unroll
+            for (int k = 0; k < Q; ++k) g[k][n] = o[k];
+        }
+    }
+    static __device__ __forceinline__ double rho_of(const M& m) { return m.rho; }
     static __device__ __forceinline__ double edge_bulk_node(const P& p, int i, int j, int cls) {
         return fp64::edge_bulk_node<FULL>(p, i, j, cls);
     }
