@@ -777,6 +777,7 @@ static int create_impl(const mrlbm_config* cfg, int precision, int device, int s
     else if (c.eq_mass_bc) h->closure = CLOSURE_RHOEQ;
     else if (c.strong_mass_bc) h->closure = CLOSURE_STRONG;
     else h->closure = CLOSURE_NONE;
+    closure_constants(h->geo, h->lat, h->closure);
     if (!make_dev_consts(h) && precision == MRLBM_FP32)
         return bail(MRLBM_EUNSUPPORTED, "FP32 closure needs equal Is/Os weight sums for every label");
 
@@ -1868,8 +1869,7 @@ int stats_in(const mrlbm_config& c, int a, int z) {
 // of shape cfg (a vector shape, or for split steps also a one-tile-per-block shape).
 void batch_items(const mrlbm_handle* h, int cfg, int aux_threads, int& aux, int& tiles, int& nbblk, int& neblk,
                  int& tiles_x) {
-    const int bn = aux_threads / 8;
-    nbblk = h->geo.nb > 0 ? (h->geo.nb + bn - 1) / bn : 1;
+    nbblk = wall_blocks(h->geo.nb, aux_threads, h->precision == MRLBM_FP64);
     neblk = (2 * h->L.nx + (h->halo_l ? 0 : h->L.ny - 2) + (h->halo_r ? 0 : h->L.ny - 2) + aux_threads - 1) / aux_threads;
     int tiles_y;
     if (is_vec_cfg(cfg)) {

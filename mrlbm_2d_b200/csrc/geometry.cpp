@@ -246,6 +246,27 @@ int build_geometry(const mrlbm_config& cfg, int nx, int ny, double x_c, double y
     return MRLBM_OK;
 }
 
+void closure_constants(Geometry& g, const Lattice64& lat, int closure) {
+    auto T = [&](int field, int l) -> double& { return g.tgeo[(size_t)field * g.nb + l]; };
+    for (int l = 0; l < g.nb; ++l) {
+        const int Is = g.tint[(size_t)I_IS * g.nb + l], Os = g.tint[(size_t)I_OS * g.nb + l];
+        double B[3] = {0, 0, 0}, F[3] = {0, 0, 0};
+        for (int k = 0; k < Q; ++k) {
+            const double hxy = T(G_HXYP + k, l);
+            const double b[3] = {4.50 * lat.w[k] * T(G_HXXP + k, l), 4.50 * lat.w[k] * T(G_HYYP + k, l), 4.50 * lat.w[k] * hxy};
+            const bool sum = closure == CLOSURE_STRONG ? (Os >> k) & 1 : closure == CLOSURE_WEAK && ((Is >> k) & 1);
+            for (int c = 0; c < 3; ++c) {
+                if (sum) B[c] = B[c] + b[c];
+                if ((Is >> k) & 1) F[c] = F[c] + b[c] * hxy;
+            }
+        }
+        for (int c = 0; c < 3; ++c) {
+            T(G_B11 + c, l) = B[c];
+            T(G_F11 + c, l) = F[c];
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------------------
 void config_defaults(mrlbm_config& c) {
     std::memset(&c, 0, sizeof c);

@@ -42,6 +42,10 @@ struct Geometry {
 int build_geometry(const mrlbm_config& cfg, int nx, int ny, double x_c, double y_c, double r_c,
                    Geometry& g, std::string& err);
 
+// The rotated closures' per-node constant sums (G_B11 .. G_F12 of the table), over the links the
+// case's closure sums them over, in its order.
+void closure_constants(Geometry& g, const Lattice64& lat, int closure);
+
 // nx, ny, centre and radius the config selects (2d_mrlbm.f90:86-92, 946-948 or explicit).
 void resolve_domain(const mrlbm_config& cfg, int& nx, int& ny, double& x_c, double& y_c, double& r_c);
 

@@ -104,7 +104,10 @@ enum GeoField : int {
     G_SCC = G_HXYP + 9,                             // stencil node m (0..7): cos^2
     G_SSS = G_SCC + 8,                              //                        sin^2
     G_SS2 = G_SSS + 8,                              //                        sin2
-    G_NFIELDS = G_SS2 + 8
+    // sums of 4.5 w_k H'_ab,k over the links the case's rotated closure sums them over, and of
+    // 4.5 w_k H'_ab,k H'_xy,k over the incoming links (constants of the node; 2d_mrlbm.f90:1700-1712)
+    G_B11 = G_SS2 + 8, G_B22, G_B12, G_F11, G_F22, G_F12,
+    G_NFIELDS
 };
 // Integer table, field-major: node i, node j, Is mask, Os mask, quadrant label, then 12
 // stencil nodes (ref points 2,3,4 x 4 corners) as i and j.

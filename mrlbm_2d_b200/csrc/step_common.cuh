@@ -194,6 +194,7 @@ constexpr int BNODES = 32;        // at most (256-thread blocks); blockDim.x / B
 constexpr int BLANES = 8;
 constexpr int G_STAGED = G_SCC;   // GeoFields 0 .. G_SCC-1 live in shared memory
 constexpr int AUX_CHUNK = 256;    // terms per warp and round in the in-order force sums
+static_assert(BLANES == wall_lanes(false), "lanes per wall node of the 8-lane blocks");
 
 template <class T>
 struct BTab {
@@ -436,6 +437,12 @@ __device__ __forceinline__ void boundary_block(const typename Phys::P& p, unsign
 template <class Phys>
 __device__ __forceinline__ void edge_block(const typename Phys::P& p, int eb, unsigned char* smem) {
     const int nx = p.L.nx, ny = p.L.ny;
+    if (p.defer && p.prev_rec && eb == p.neblk - 1) {
+        // a block of its own for the in-order sums: behind an edge node's chain they made the last edge
+        // block of a 400 x 100 step take 4.7 us where the others took 1.6
+        record_sums(p.prev_partials, p.nb, ny, p.halo_l, p.prev_rec, p.prev_iter, smem);
+        return;
+    }
     const StepRec sr = step_rec(p);
     const int e = eb * (int)blockDim.x + (int)threadIdx.x;
     const int cl = p.halo_l ? 0 : 1, cr = p.halo_r ? 0 : 1;         // edge columns of this lattice
@@ -453,23 +460,31 @@ __device__ __forceinline__ void edge_block(const typename Phys::P& p, int eb, un
         if (sr.do_stats && i == 1 && !p.halo_l) p.partials[2 * p.nb + j - 1] = rho;
     }
     if (!p.defer) inlet_tail<Phys>(p, sr, smem, eb);
-    else if (eb == 0 && p.prev_rec) record_sums(p.prev_partials, p.nb, p.L.ny, p.halo_l, p.prev_rec, p.prev_iter, smem);
 }
 
-// Shared memory of an auxiliary block: the boundary tables and, afterwards, the tail's
-// staged terms.
+// Shared memory of an auxiliary block: the 8-lane boundary tables, or the 16-lane wall blocks' per-node
+// scratch, and afterwards the tail's staged terms.
+constexpr int WALL_TERMS = 5;     // rows of nine per-direction terms per node (wall_block)
 template <class T>
 constexpr int aux_smem_bytes() {
-    return (int)(sizeof(T) * G_STAGED + sizeof(int) * I_NFIELDS) * BNODES > 3 * AUX_CHUNK * (int)sizeof(double)
-               ? (int)(sizeof(T) * G_STAGED + sizeof(int) * I_NFIELDS) * BNODES
-               : 3 * AUX_CHUNK * (int)sizeof(double);
+    const int wall = sizeof(T) == 8 ? WALL_TERMS * Q * 16 * (int)sizeof(T)
+                                    : (int)(sizeof(T) * G_STAGED + sizeof(int) * I_NFIELDS) * BNODES;
+    const int sums = 3 * AUX_CHUNK * (int)sizeof(double);
+    return wall > sums ? wall : sums;
 }
 
 // Auxiliary work item b of a step: boundary block b (b < nbblk) or edge block b - nbblk.
-template <class Phys, bool WIDE, bool WAIT = true>
+// WAIT: the item waits for the previous step itself, a wall block after loading its tables;
+// otherwise the kernel waited before calling it.
+template <class Phys, bool WIDE, bool WAIT>
 __device__ __forceinline__ void aux_item(const typename Phys::P& p, unsigned char* smem, int b) {
-    if (b < p.nbblk) boundary_block<Phys, WIDE, WAIT>(p, smem, b);
-    else edge_block<Phys>(p, b - p.nbblk, smem);
+    if (b < p.nbblk) {
+        if constexpr (Phys::WALL_LANES == 16) Phys::template wall_block<WAIT>(p, smem, b);
+        else boundary_block<Phys, WIDE, WAIT>(p, smem, b);
+    } else {
+        if (WAIT) wait_prior_grid();
+        edge_block<Phys>(p, b - p.nbblk, smem);
+    }
 }
 
 // Whether a kernel of `threads` threads and `minb` resident blocks per SM takes the wide wall path.
@@ -493,8 +508,7 @@ constexpr int AUX_THREADS = 128;
 template <class Phys>
 __global__ void __launch_bounds__(AUX_THREADS) aux_kernel(const __grid_constant__ typename Phys::P p) {
     __shared__ __align__(16) unsigned char smem[aux_smem_bytes<typename Phys::T>()];
-    wait_prior_grid();
-    aux_item<Phys, true, false>(p, smem, (int)blockIdx.x);
+    aux_item<Phys, true, true>(p, smem, (int)blockIdx.x);
 }
 
 // Start of a bulk launch: let the next launch (the next step's auxiliary blocks) be scheduled.
@@ -514,13 +528,12 @@ __device__ __forceinline__ void bulk_end(const StepParams<T>& p) {
 template <class P>
 inline int edge_blocks(const P& p, int nthr) {
     const int n = 2 * p.L.nx + (p.halo_l ? 0 : p.L.ny - 2) + (p.halo_r ? 0 : p.L.ny - 2);
-    return (n + nthr - 1) / nthr;
+    return (n + nthr - 1) / nthr + (p.defer && p.prev_rec ? 1 : 0);
 }
 
 template <class Phys>
 inline int launch_aux(typename Phys::P p, cudaStream_t s) {
-    const int bn = AUX_THREADS / BLANES;
-    p.nbblk = p.nb > 0 ? (p.nb + bn - 1) / bn : 1;
+    p.nbblk = wall_blocks(p.nb, AUX_THREADS, sizeof(typename Phys::T) == 8);
     p.neblk = edge_blocks(p, AUX_THREADS);
     return launch_after_prior(aux_kernel<Phys>, (unsigned)(p.nbblk + p.neblk), AUX_THREADS, 0, s, p) == cudaSuccess ? 0 : -1;
 }
@@ -857,8 +870,7 @@ int launch_step_tiles(typename Phys::P p, cudaStream_t s) {
     const long long nblocks = (long long)p.tiles_x * tiles_y;
     p.tx_magic = tile_div_magic(p.tiles_x, nblocks);
     if constexpr (Phys::FUSED_AUX) {
-        const int bn = nthr / BLANES;
-        p.nbblk = p.nb > 0 ? (p.nb + bn - 1) / bn : 1;
+        p.nbblk = wall_blocks(p.nb, nthr, sizeof(typename Phys::T) == 8);
         p.neblk = edge_blocks(p, nthr);
         return launch_after_prior(step_kernel_fused<Phys, BX, BY, NJ, MINB>, (unsigned)(p.nbblk + p.neblk + nblocks), nthr,
                                   0, s, p) == cudaSuccess

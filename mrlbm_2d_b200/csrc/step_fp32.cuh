@@ -541,6 +541,7 @@ struct PhysicsT {
         fp32::boundary_close<FULL, true>(p, tb, li, l, g, ux2, uy2, mx2, my2, ux3, uy3, mx3, my3, Fx, Fy);
     }
     // registers per thread a kernel needs before its wall node's populations are gathered ahead
+    static constexpr int WALL_LANES = 8;
     static constexpr int WIDE_REGS = 96;
     // One launch per step with tile shapes: the FP32 wall closures fit the tiles' register
     // budgets, so the wall and edge blocks run as the first blocks of the bulk grid.

@@ -78,10 +78,13 @@ template <class Phys>
 __global__ void __launch_bounds__(AUX_THREADS) pair_first(const __grid_constant__ typename Phys::P p,
                                                           const __grid_constant__ PairBand band, const PairRect core) {
     __shared__ __align__(16) unsigned char smem[aux_smem_bytes<typename Phys::T>()];
-    wait_prior_grid();
     const int b = (int)blockIdx.x, na = p.nbblk + p.neblk;
-    if (b < na) aux_item<Phys, true, false>(p, smem, b);
-    else band_node<Phys, true>(p, band, core, (b - na) * AUX_THREADS + (int)threadIdx.x);
+    if (b < na) {
+        aux_item<Phys, true, true>(p, smem, b);
+        return;
+    }
+    wait_prior_grid();
+    band_node<Phys, true>(p, band, core, (b - na) * AUX_THREADS + (int)threadIdx.x);
 }
 
 // Shared-memory ring of a block of the two-step tiles: a slot holds one row of all nine planes, as
@@ -293,9 +296,12 @@ __global__ void __launch_bounds__(WARPS * 32, MINB) pair_second(const __grid_con
         pair_tile<Phys, WARPS, NS, STAGES, FULL>(p, pair_smem, core, b - na, strips, chunks, flip);
         return;
     }
+    if (b < na) {
+        aux_item<Phys, wide_wall<Phys>(WARPS * 32, MINB), true>(p, pair_smem, b);
+        return;
+    }
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (b < na) aux_item<Phys, wide_wall<Phys>(WARPS * 32, MINB), false>(p, pair_smem, b);
-    else band_node<Phys, false>(p, band, core, (b - na - nt) * WARPS * 32 + (int)threadIdx.x);
+    band_node<Phys, false>(p, band, core, (b - na - nt) * WARPS * 32 + (int)threadIdx.x);
 }
 
 // Band of an auxiliary launch: rings of width w and the rectangle clipped clear of them.
@@ -325,14 +331,13 @@ int launch_pair(typename Phys::P p1, typename Phys::P p2, const PairPlan& plan, 
         if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(R)) != cudaSuccess) return -1;
         if (dev < 64) attr_set |= 1ull << dev;
     }
-    auto wall_blocks = [](const typename Phys::P& p, int nthr) { return p.nb > 0 ? (p.nb + nthr / BLANES - 1) / (nthr / BLANES) : 1; };
-    p1.nbblk = wall_blocks(p1, AUX_THREADS);
+    p1.nbblk = wall_blocks(p1.nb, AUX_THREADS, sizeof(T) == 8);
     p1.neblk = edge_blocks(p1, AUX_THREADS);
     const PairBand b1 = pair_band(2, plan.halo, nx, ny), b2 = pair_band(1, plan.core, nx, ny);
     const int n1 = p1.nbblk + p1.neblk + (band_nodes(b1, nx, ny) + AUX_THREADS - 1) / AUX_THREADS;
     if (launch_after_prior(pair_first<Phys>, (unsigned)n1, AUX_THREADS, 0, s, p1, b1, plan.core) != cudaSuccess) return -1;
     const int strips = (nx - 4 + PAIR_COLS - 1) / PAIR_COLS;
-    p2.nbblk = wall_blocks(p2, WARPS * 32);
+    p2.nbblk = wall_blocks(p2.nb, WARPS * 32, sizeof(T) == 8);
     p2.neblk = edge_blocks(p2, WARPS * 32);
     p2.tmap = p1.tmap;                                     // of level n
     const int n2 = p2.nbblk + p2.neblk + (strips + WARPS * NS - 1) / (WARPS * NS) * plan.chunks +

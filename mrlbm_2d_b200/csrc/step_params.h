@@ -60,7 +60,8 @@ struct alignas(64) StepParams {
     int do_stats;                 // stats step: forces + inlet density sum
     // curved wall
     int nb, nbblk;                // boundary nodes, boundary blocks at the start of the grid
-    int neblk;                    // edge blocks (one thread per domain-edge node) after them
+    int neblk;                    // edge blocks (one thread per domain-edge node) after them, and with a deferred
+                                  // record to sum (prev_rec) one more that does it
     int halo_l, halo_r;           // x-slab of a larger domain: column 0 / nx+1 hold the neighbour's populations
     const int* __restrict__ bint; // IntField table [I_NFIELDS * nb]
     const T* __restrict__ bgeo;   // GeoField table [G_NFIELDS * nb]
@@ -73,7 +74,7 @@ struct alignas(64) StepParams {
     unsigned* counter;            // [0] arrivals of boundary blocks, [1] of inlet edge blocks (reset by the last)
     double* rec;                  // REC_WORDS doubles for this step, or null
     // Deferred record sums (single-case steps): with defer set, a stats step leaves its terms in
-    // `partials` and no block of it waits for the others to sum them; the next launch's first
+    // `partials` and no block of it waits for the others to sum them; the next launch's last
     // edge block (or the finishing kernel, launch_finish_record) sums them in index order into
     // prev_rec, taking the in-order sums off the step's critical path.
     int defer;
@@ -202,6 +203,14 @@ inline bool is_vec_cfg(int c) { return c >= VEC_CFG0 && c < PIPE_CFG0; }
 // Kernel launches of one time step: FP32 tile shapes run the step as one launch (the wall and
 // edge blocks first in the grid), every other shape as an auxiliary launch and a bulk launch.
 inline int step_launches(bool fp32, int c) { return fp32 && c >= 0 && c < N_TILE_CFGS ? 1 : 2; }
+
+// Lanes per curved-wall node of the wall blocks: 16 in FP64 (wall_block, step_fp64.cuh), 8 in FP32
+// (boundary_block, step_common.cuh), and the wall blocks of `threads` threads for nb nodes (one at least).
+constexpr int wall_lanes(bool fp64) { return fp64 ? 16 : 8; }
+inline int wall_blocks(int nb, int threads, bool fp64) {
+    const int per = threads / wall_lanes(fp64);
+    return nb > 0 ? (nb + per - 1) / per : 1;
+}
 
 // Host-side launch entry points (step_f64.cu / step_f32.cu).  `workers` is the persistent
 // CTA count for TMA shapes (ignored otherwise).  Return 0, -1 on a launch error, -2 when the
