@@ -214,7 +214,7 @@ __device__ __forceinline__ Mac node_macro(const P& p, int i, int j, const double
 __device__ __forceinline__ void stencil_node(const P& p, int si, int sj, double cc, double ss, double s2, double& ux,
                                              double& uy, double& mx, double& my) {
     double f[Q];
-    gather(p, si, sj, f);
+    gather_interior(p, si, sj, f);                  // stencil nodes are interior fluid nodes (checked at setup)
     const Mac m = moments(f, p.hm, p.hp);
     ux = m.ux;
     uy = m.uy;
@@ -271,9 +271,14 @@ static __device__ __noinline__ void closure_unrotated(const P& p, const BTab<dou
     m.mxy = Mxy;
 }
 
-// Collision and reconstruction of direction k alone: collide's expressions with this direction's signs
-// and tables (adding a zero where a direction has no such term changes no bit).
-__device__ __forceinline__ double collide_dir(const P& p, const Mac& m, int k) {
+// One direction's constants: velocity components, H_xx and H_yy values, weight.
+struct Dir { double x, y, hx, hy, w; };
+
+// Collision and reconstruction of one direction: collide's expressions with this direction's signs
+// (3 (x u + y v) is its +-t1 .. +-t8, x y its +-c; products with 0 and +-1 are exact, and adding a zero
+// where a direction has no such term changes no bit).  No branch depends on the direction: with the
+// nine cases spelled out the lanes of a node took them one after another (1900 cycles of 6400).
+__device__ __forceinline__ double collide_dir(const P& p, const Mac& m, const Dir& e) {
     const double om = p.omega, om1 = p.omega1;
     double mxx = om1 * m.mxx + om * m.ux * m.ux;
     double myy = om1 * m.myy + om * m.uy * m.uy;
@@ -284,12 +289,8 @@ __device__ __forceinline__ double collide_dir(const P& p, const Mac& m, int k) {
         myy = myy - t;
     }
     const double a = 4.50 * mxx, b = 4.50 * myy, c = 9.00 * mxy;
-    const double alpha = a * (ex(k) != 0 ? p.hp : p.hm), beta = b * (ey(k) != 0 ? p.hp : p.hm);
-    const double t1 = 3.0 * m.ux, t2 = 3.0 * m.uy, t5 = 3.0 * (m.ux + m.uy), t8 = 3.0 * (m.ux - m.uy);
-    const double t = k == 0 ? 0.0 : k == 1 ? t1 : k == 2 ? t2 : k == 3 ? -t1 : k == 4 ? -t2 : k == 5 ? t5 : k == 6 ? -t8 : k == 7 ? -t5 : t8;
-    const double d = k < 5 ? 0.0 : (k & 1) ? c : -c;
-    const double w = (k == 0 ? p.w[0] : k < 5 ? p.w[1] : p.w[5]) * m.rho;
-    return w * ((((1.0 + t) + alpha) + beta) + d);
+    const double t = 3.0 * (e.x * m.ux + e.y * m.uy);
+    return (e.w * m.rho) * ((((1.0 + t) + a * e.hx) + b * e.hy) + (e.x * e.y) * c);
 }
 
 // Wall block: curved-wall nodes (2d_mrlbm.f90:294-311 and the routines it calls) by 16 lanes each.  Lane s
@@ -312,6 +313,7 @@ __device__ __forceinline__ void wall_block(const P& p, unsigned char* smem, int 
     const int k = min(lane, Q - 1), s = lane & 7, r = s >> 2;      // direction; stencil node, reference point 2 + r
     const bool dir = lane < Q;
     const int ekx = ex(k), eky = ey(k);
+    const Dir e{(double)ekx, (double)eky, ekx != 0 ? p.hp : p.hm, eky != 0 ? p.hp : p.hm, k == 0 ? p.w[0] : k < 5 ? p.w[1] : p.w[5]};
     const int closure = p.closure;
     const bool rotated = closure != CLOSURE_UNROTATED;
     const bool interp = !rotated || p.vel_interp || p.mom_interp;
@@ -375,7 +377,7 @@ __device__ __forceinline__ void wall_block(const P& p, unsigned char* smem, int 
         // numerical_boundary_cases_rotation (strong, 2d_mrlbm.f90:1635-1765), _weak (1767-1871), _rhoeq (1873-1972)
         const double uxp = m.ux * cth + m.uy * sth;                              // 2d_mrlbm.f90:304-305
         const double uyp = m.uy * cth - m.ux * sth;
-        const double omega = p.omega, wk = k == 0 ? p.w[0] : k < 5 ? p.w[1] : p.w[5];
+        const double omega = p.omega, wk = e.w;
         const double A_i = wk * (1.0 + 3.0 * uxp * cxp + 3.0 * uyp * cyp);
         const double E_i = wk * (1.0 + 3.0 * uxp * cxp + 3.0 * uyp * cyp + 4.50 * (uxp * uxp) * hxx +
                                  4.50 * (uyp * uyp) * hyy + 9.0 * (uxp * uyp) * hxy);
@@ -423,20 +425,22 @@ __device__ __forceinline__ void wall_block(const P& p, unsigned char* smem, int 
         m.myy = Mxx * ssth + Myy * ccth + Mxy * s2th;
         m.mxy = (Mxx - Myy) * 0.50 * s2th + Mxy * c2th;
     }
-    const double fo = collide_dir(p, m, k);
+    const double fo = collide_dir(p, m, e);
     if (active && dir) p.dst[(int64_t)k * p.L.plane + (int64_t)nj * p.L.pitch + ni + p.L.off] = fo;
     // momentum-exchange force (evaluate_forces, 2d_mrlbm.f90:558-591): lanes 0 and 1 sum the outgoing
     // populations' x and y, lanes 2 and 3 the incoming ones'
     __syncwarp();
     if (dir) {
-        sm[k] = out ? fo : 0.0;
-        sm[Q + k] = in ? fk : 0.0;
+        sm[k] = out ? fo * e.x : 0.0;
+        sm[Q + k] = out ? fo * e.y : 0.0;
+        sm[2 * Q + k] = in ? fk * e.x : 0.0;
+        sm[3 * Q + k] = in ? fk * e.y : 0.0;
     }
     __syncwarp();
     double sum = 0.0;
-    const double* row = sm + ((lane >> 1) & 1) * Q;
+    const double* row = sm + (lane & 3) * Q;
 #pragma unroll
-    for (int q = 0; q < Q; ++q) sum = sum + row[q] * (double)((lane & 1) ? ey(q) : ex(q));
+    for (int q = 0; q < Q; ++q) sum = sum + row[q];
     const double F = __shfl_down_sync(all, sum, 2, 16) - sum;
     if (active && lane < 2) {
         if (sr.do_stats) p.partials[lane * nb + l] = F;
