@@ -77,6 +77,14 @@ MRLBM_HD SrcSlot stream_source(int nx, int ny, int i, int j, int k, bool xper, b
     return s;
 }
 
+// Threads of the edge blocks' enumeration (edge_block, step_common.cuh): column 1, column nx, row 1 and row
+// ny without the corners, each group rounded up to whole warps so that no warp mixes two kinds of
+// edge.  An x-slab's halo faces are not edges.
+MRLBM_HD int edge_pad(int n) { return (n + 31) & ~31; }
+MRLBM_HD int edge_threads(int nx, int ny, bool hl, bool hr) {
+    return (hl ? 0 : edge_pad(ny)) + (hr ? 0 : edge_pad(ny)) + 2 * edge_pad(nx - (hl ? 0 : 1) - (hr ? 0 : 1));
+}
+
 // Node class inside the cylinder bounding box (values >= 0 are boundary-node indices).
 constexpr int CLS_FLUID = -1;
 constexpr int CLS_SOLID = -2;

@@ -79,6 +79,39 @@ __device__ __forceinline__ void gather(const StepParams<T>& p, int i, int j, T f
     }
 }
 
+// f(i,j,:) of an edge node, or of the outlet column's neighbour: stream_source's cases as selects on the
+// offset from the node's own slot, so the nine loads leave together (with the branches of `gather`
+// an edge warp spent 2600 cycles before its closure).
+template <class T>
+__device__ __forceinline__ void edge_gather(const StepParams<T>& p, int i, int j, T f[Q]) {
+    const int nx = p.L.nx, ny = p.L.ny, pitch = p.L.pitch, plane = (int)p.L.plane;
+    const bool top = j == ny, bottom = j == 1, left = i == 1 && !p.halo_l, right = i == nx && !p.halo_r;
+    const bool slip = p.freeslip && !p.yper;
+    const T* s = p.src + (j * pitch + i + p.L.off);
+#pragma unroll
+    for (int k = 0; k < Q; ++k) {
+        const bool xhit = ex(k) > 0 ? left : ex(k) < 0 ? right : false;
+        const int wrap = ex(k) > 0 ? nx - 1 : 1 - nx;               // the other end of the row, from here
+        const int pulled = k * plane - ey(k) * pitch - ex(k);
+        int o = xhit && p.xper ? k * plane + wrap : pulled;
+        if (ey(k) != 0) {
+            const bool yhit = ey(k) > 0 ? bottom : top;
+            const int m = mirror_y(k) * plane;
+            const int reflected = !xhit ? m - ex(k) : p.xper ? m + wrap : pulled;
+            if (yhit && slip) o = reflected;
+            if (yhit && p.yper) o = k * plane + (ey(k) > 0 ? ny - 1 : 1 - ny) * pitch;
+        }
+        f[k] = __ldg(s + o);
+    }
+    for (int q = 0; q < p.n_ovr; ++q)                               // by a select over the nine, as in `gather`
+        if (p.ovr[q].i == i && p.ovr[q].j == j) {
+            const int kq = p.ovr[q].k;
+            const T v = (T)p.ovr[q].v;
+#pragma unroll
+            for (int k = 0; k < Q; ++k) f[k] = k == kq ? v : f[k];
+        }
+}
+
 // Non-positive (or NaN) density at a node: set the handle's error flag.  The flag is read
 // first, so a case that has gone unstable costs one atomic per SM until the flag is visible,
 // not one per node and step on a single address.
@@ -446,16 +479,20 @@ __device__ __forceinline__ void edge_block(const typename Phys::P& p, int eb, un
     const StepRec sr = step_rec(p);
     const int e = eb * (int)blockDim.x + (int)threadIdx.x;
     const int cl = p.halo_l ? 0 : 1, cr = p.halo_r ? 0 : 1;         // edge columns of this lattice
-    const int nl = cl * ny, nr = cr * ny, nrow = nx - cl - cr;
-    if (e < nl + nr + 2 * nrow) {
-        int i, j;
-        if (e < nl) { i = 1; j = e + 1; }
-        else if (e < nl + nr) { i = nx; j = e - nl + 1; }
-        else {
-            const int q = e - nl - nr;
-            i = cl + 1 + (q < nrow ? q : q - nrow);
-            j = q < nrow ? 1 : ny;
-        }
+    const int nl = cl * edge_pad(ny), nr = cr * edge_pad(ny), nrow = nx - cl - cr, rp = edge_pad(nrow);
+    int i, j;
+    bool on;
+    if (e < nl + nr) {
+        i = e < nl ? 1 : nx;
+        j = 1 + (e < nl ? e : e - nl);
+        on = j <= ny;
+    } else {
+        const int q = e - nl - nr, side = q >= rp;
+        i = cl + 1 + (q - side * rp);
+        j = side ? ny : 1;
+        on = q < 2 * rp && i <= cl + nrow;
+    }
+    if (on) {
         const double rho = Phys::edge_bulk_node(p, i, j, CLS_FLUID);
         if (sr.do_stats && i == 1 && !p.halo_l) p.partials[2 * p.nb + j - 1] = rho;
     }
@@ -527,8 +564,7 @@ __device__ __forceinline__ void bulk_end(const StepParams<T>& p) {
 
 template <class P>
 inline int edge_blocks(const P& p, int nthr) {
-    const int n = 2 * p.L.nx + (p.halo_l ? 0 : p.L.ny - 2) + (p.halo_r ? 0 : p.L.ny - 2);
-    return (n + nthr - 1) / nthr + (p.defer && p.prev_rec ? 1 : 0);
+    return (edge_threads(p.L.nx, p.L.ny, p.halo_l, p.halo_r) + nthr - 1) / nthr + (p.defer && p.prev_rec ? 1 : 0);
 }
 
 template <class Phys>

@@ -128,9 +128,10 @@ constexpr int M_INLET = (1 << 0) | (1 << 2) | (1 << 3) | (1 << 4) | (1 << 6) | (
 constexpr int M_TOP = (1 << 0) | (1 << 1) | (1 << 2) | (1 << 3) | (1 << 5) | (1 << 6);
 constexpr int M_BOTTOM = (1 << 0) | (1 << 1) | (1 << 3) | (1 << 4) | (1 << 7) | (1 << 8);
 
-// Edge nodes: Dirichlet values and the regularized edge closures of apply_bc /
+// Edge nodes (gn: the populations of node (nx - 1, j) at the outlet): Dirichlet values and the
+// regularized edge closures of apply_bc /
 // apply_bc_incomp (2d_mrlbm.f90:249-272, 1237-1494) in deviation form.
-__device__ __forceinline__ void edge_node(const P& p, int i, int j, const float g[Q], Mac& m) {
+__device__ __forceinline__ void edge_node(const P& p, int i, int j, const float g[Q], const float gn[Q], Mac& m) {
     const int nx = p.L.nx, ny = p.L.ny;
     const bool outlet = !p.xper && !p.halo_r && i == nx;
     const bool inlet = !p.xper && !p.halo_l && i == 1;
@@ -138,8 +139,6 @@ __device__ __forceinline__ void edge_node(const P& p, int i, int j, const float 
     const bool bottom = p.walls_ref && j == 1;
     const DevConsts& c = p.dc;
     if (outlet) {                                   // rho, u copied from column nx-1
-        float gn[Q];
-        gather(p, nx - 1, j, gn);
         const Mac mn = moments(p, gn);
         m.drho = mn.drho; m.rho = mn.rho; m.ux = mn.ux; m.uy = mn.uy;
     }
@@ -444,10 +443,11 @@ __device__ __forceinline__ void boundary_close(const P& p, const BTab<float>& tb
 // registers and the gathers of a node overlap.
 template <bool FULL>
 __device__ __forceinline__ double edge_bulk_node(const P& p, int i, int j, int cls) {
-    float g[Q];
-    gather(p, i, j, g);
+    float g[Q], gn[Q];
+    edge_gather(p, i, j, g);
+    if (i == p.L.nx && !p.halo_r) edge_gather(p, i - 1, j, gn);       // the outlet's neighbour, in the same round trip
     Mac m = moments(p, g);
-    edge_node(p, i, j, g, m);
+    edge_node(p, i, j, g, gn, m);
     if ((cls == CLS_SOLID && p.zero_solid_u) || cls == CLS_SOLID_ZERO) { m.ux = 0.f; m.uy = 0.f; }
     if (!(m.rho > 0.0f)) flag_bad_density(p);
     if (FULL && p.macro) store_macro(p, i, j, 1.0 + (double)m.drho, m.ux, m.uy, m.mxx, m.myy, m.mxy);

@@ -107,19 +107,16 @@ constexpr int M_INLET = (1 << 0) | (1 << 2) | (1 << 3) | (1 << 4) | (1 << 6) | (
 constexpr int M_TOP = (1 << 0) | (1 << 1) | (1 << 2) | (1 << 3) | (1 << 5) | (1 << 6);
 constexpr int M_BOTTOM = (1 << 0) | (1 << 1) | (1 << 3) | (1 << 4) | (1 << 7) | (1 << 8);
 
-// Edge nodes: Dirichlet values (2d_mrlbm.f90:249-272) then the regularized closure the
+// Edge nodes (fn: the populations of node (nx - 1, j) at the outlet, whose moments it copies): Dirichlet
+// values (2d_mrlbm.f90:249-272) then the regularized closure the
 // reference applies last at this node (apply_bc / apply_bc_incomp, 2d_mrlbm.f90:313-351).
-__device__ __forceinline__ void edge_node(const P& p, int i, int j, const double f[Q], Mac& m) {
+__device__ __forceinline__ void edge_node(const P& p, int i, int j, const double f[Q], const double fn[Q], Mac& m) {
     const int nx = p.L.nx, ny = p.L.ny;
     const bool outlet = !p.xper && !p.halo_r && i == nx;
     const bool inlet = !p.xper && !p.halo_l && i == 1;
     const bool top = p.walls_ref && j == ny;
     const bool bottom = p.walls_ref && j == 1;
-    if (outlet) {
-        double fn[Q];
-        gather(p, nx - 1, j, fn);
-        moments_u(fn, m.rho, m.ux, m.uy);
-    }
+    if (outlet) moments_u(fn, m.rho, m.ux, m.uy);
     if (inlet) {
         m.ux = p.u_in ? p.u_in[j - 1] : p.uinlet;
         m.uy = p.vinlet;
@@ -203,7 +200,11 @@ __device__ __forceinline__ void collide(const P& p, const Mac& m, double fo[Q]) 
 // Post-boundary-condition macroscopic values of a non-cylinder node.
 __device__ __forceinline__ Mac node_macro(const P& p, int i, int j, const double f[Q]) {
     Mac m = moments(f, p.hm, p.hp);
-    if (!is_interior(p, i, j)) edge_node(p, i, j, f, m);
+    if (!is_interior(p, i, j)) {
+        double fn[Q];
+        edge_gather(p, max(i - 1, 1), j, fn);           // the outlet's neighbour
+        edge_node(p, i, j, f, fn, m);
+    }
     return m;
 }
 
@@ -458,10 +459,11 @@ __device__ __forceinline__ void wall_block(const P& p, unsigned char* smem, int 
 // branch of their own, so the bulk path's registers are not affected).
 template <bool FULL>
 __device__ __forceinline__ double edge_bulk_node(const P& p, int i, int j, int cls) {
-    double f[Q];
-    gather(p, i, j, f);
+    double f[Q], fn[Q];
+    edge_gather(p, i, j, f);
+    if (i == p.L.nx && !p.halo_r) edge_gather(p, i - 1, j, fn);       // the outlet's neighbour, in the same round trip
     Mac m = moments(f, p.hm, p.hp);
-    edge_node(p, i, j, f, m);
+    edge_node(p, i, j, f, fn, m);
     if ((cls == CLS_SOLID && p.zero_solid_u) || cls == CLS_SOLID_ZERO) { m.ux = 0.0; m.uy = 0.0; }
     if (!(m.rho > 0.0)) flag_bad_density(p);
     if (FULL && p.macro) store_macro(p, i, j, m.rho, m.ux, m.uy, m.mxx, m.myy, m.mxy);
