@@ -28,6 +28,10 @@ using namespace mrlbm;
 namespace {
 thread_local std::string g_create_error;
 constexpr int RING_CAP = 8192;                // stats records buffered on the device
+// Steps per replayed run (step_replay), longest first, and the graphs a handle keeps: both lengths from
+// either time level.
+constexpr int REPLAY_STEPS[2] = {64, 16};
+constexpr int N_REPLAYS = 4;
 constexpr int STREAMS_MAX_STEPS = 1024;       // steps per launch of the per-case streams schedule
 }
 
@@ -53,7 +57,7 @@ struct mrlbm_handle {
     void* d_bgeo = nullptr;
     int* d_bint = nullptr;
     int* d_boxmap = nullptr;
-    double* d_partials = nullptr;             // two slots of the per-step record terms
+    double* d_partials = nullptr;             // slots of the per-step record terms: 0, 1 launched steps, 2, 3 replayed
     size_t partials_n = 0;                    // doubles per slot
     int pslot = 0;                            // slot the next stats step writes
     // a stats step whose record sums are deferred to the next launch (StepParams::defer)
@@ -93,6 +97,17 @@ struct mrlbm_handle {
     DevConsts dc{};
     bool host_only = false;
     std::vector<float> geo32;                 // FP32 tables of a host-only FP32 handle
+    // runs of steps captured into graphs and replayed (step_replay)
+    struct Replay {
+        cudaGraphExec_t exec = nullptr;
+        int steps = 0, launches = 0;
+        std::vector<uintptr_t> sig;           // everything the captured launches hold that can change
+        uint64_t used = 0;
+    } replay[N_REPLAYS];
+    uint64_t replay_clock = 0;
+    int64_t stepped = 0;                      // steps taken by the handle
+    bool no_replay = false;                   // autotuner trials of single shapes
+    int* d_call = nullptr;                    // call state of the replay (StepParams::call)
     std::vector<OvrEntry> ovr;                // loaded-state overrides (see OvrEntry)
     bool ovr_live = false;                    // true until the first step after a load
     OvrEntry* d_ovr = nullptr;
@@ -581,24 +596,39 @@ bool pair_ok(const mrlbm_handle* h) {
            !(h->surf_on && (stats_at(h, a) || stats_at(h, b)));
 }
 
+// Parameters of a step of the handle but for its time levels and record.
+template <class T>
+StepParams<T> case_params(mrlbm_handle* h) {
+    StepParams<T> p{};
+    fill_common(h, p);
+    p.u_in = h->has_uin ? (const T*)h->d_uin : nullptr;
+    p.body = h->has_body ? (const T*)h->d_body : nullptr;
+    return p;
+}
+
+template <class T>
+int launch_pair_params(mrlbm_handle* h, int cur, StepParams<T> (&p)[2], cudaStream_t st) {
+    p[0].src = (const T*)h->buf[cur];
+    p[0].dst = (T*)h->mid;
+    p[0].tmap = h->tmap_pair[cur];
+    p[1].src = (const T*)h->mid;
+    p[1].dst = (T*)h->buf[1 - cur];
+    if constexpr (sizeof(T) == 8) return launch_pair_f64(p[0], p[1], h->plan, cur != 0, st);
+    else return launch_pair_f32(p[0], p[1], h->plan, cur != 0, st);
+}
+
 template <class T>
 int launch_pair_t(mrlbm_handle* h) {
     StepParams<T> p[2];
     for (int q = 0; q < 2; ++q) {
         const int iter = h->iter + 1 + q;
         const bool stats = stats_at(h, iter);
-        p[q] = StepParams<T>{};
-        fill_common(h, p[q]);
+        p[q] = case_params<T>(h);
         set_deferred(h, p[q]);
-        p[q].src = (const T*)(q == 0 ? h->buf[h->cur] : h->mid);
-        p[q].dst = (T*)(q == 0 ? h->mid : h->buf[1 - h->cur]);
-        p[q].u_in = h->has_uin ? (const T*)h->d_uin : nullptr;
-        p[q].body = h->has_body ? (const T*)h->d_body : nullptr;
         p[q].zero_solid_u = plot_at(h, iter);
         p[q].do_stats = stats;
         p[q].rec = stats ? h->d_ring + (size_t)h->ring_n * REC_WORDS : nullptr;
         p[q].iter = iter;
-        if (q == 0) p[q].tmap = h->tmap_pair[h->cur];
         p[q].fstat = fields_at(h, iter) ? h->d_fstat : nullptr;
         h->pend.on = false;
         if (stats) {
@@ -608,8 +638,7 @@ int launch_pair_t(mrlbm_handle* h) {
         }
         if (p[q].fstat) ++h->fstat_n;
     }
-    if constexpr (sizeof(T) == 8) return launch_pair_f64(p[0], p[1], h->plan, h->cur != 0, h->stream);
-    else return launch_pair_f32(p[0], p[1], h->plan, h->cur != 0, h->stream);
+    return launch_pair_params<T>(h, h->cur, p, h->stream);
 }
 
 int launch_two(mrlbm_handle* h) {
@@ -624,12 +653,153 @@ int launch_two(mrlbm_handle* h) {
     return MRLBM_OK;
 }
 
+// Replayed runs.  Launched one by one, the kernels of a step reach the GPU 1.9 to 2.5 us apart; as nodes of
+// a graph (with the same programmatic dependence) 1.0 us apart.  That bounds a step whose work is
+// shorter than its launches.  A run of REPLAY_STEPS steps is captured once per start level and
+// replayed; what differs from replay to replay (iteration, ring slot, the record still to be summed) comes
+// from the call state, copied ahead of it.  Calls of 400 steps and the read of their forces, us, launched
+// and replayed: 80 x 50 FP64 2100, 1620; 400 x 100 2100, 1690 (FP32 1520, 1395); 1003 x 251 2690, 2420
+// (FP32 2295, 2210); 1400 x 350 the same, its steps outlast their launches.
+constexpr int64_t REPLAY_MAX_NODES = 400000;
+
+// Length of the run to replay for the next `left` steps, or 0: launched steps.  Every step of the run must be
+// one whose launch differs from its captured form in the call state only.
+int replay_length(const mrlbm_handle* h, int left) {
+    if (left < REPLAY_STEPS[1] || h->no_replay || h->ovr_live || h->surf_on || !h->own_stream || is_tma_cfg(h->tile_cfg) ||
+        (int64_t)h->L.nx * h->L.ny > REPLAY_MAX_NODES || h->halo_l || h->halo_r)
+        return 0;
+    const mrlbm_config& c = h->cfg;
+    for (int n : REPLAY_STEPS) {
+        const int a = h->iter + 1, z = h->iter + n;
+        if (left < n || h->ring_n + n > RING_CAP) continue;
+        // a graph costs its first call about as much as 2 n launched steps would take: not for calls or
+        // handles that end before it has paid (0.3 ms for 16 and 0.6 ms for 64 steps, measured)
+        if (left < 3 * n && h->stepped < 8 * n) continue;
+        const bool fields = h->d_fstat && std::max(a, h->fstat_begin) <= std::min(z, h->fstat_end);
+        if (fields && !(h->fstat_begin <= a && z <= h->fstat_end)) continue;       // all of the run or none of it
+        // a plot step's solid velocities follow the call state in the tile shapes only
+        if (h->tile_cfg >= N_TILE_CFGS && plot_at(h, 0) && (a <= 0 || z / c.iplot > h->iter / c.iplot)) continue;
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();
+            return 0;                                              // the caller is capturing: plain launches
+        }
+        return n;
+    }
+    return 0;
+}
+
+template <class T>
+int capture_run(mrlbm_handle* h, int n, bool fields, cudaStream_t st) {
+    const mrlbm_config& c = h->cfg;
+    int cur = h->cur;
+    auto params = [&](int s) {
+        StepParams<T> p = case_params<T>(h);
+        p.call = h->d_call;
+        p.bstep = s;
+        p.stats_lo = c.post_process ? c.statsbegin : 1;
+        p.stats_hi = c.post_process ? c.statsend : 0;
+        p.ring = h->d_ring;
+        p.plot_every = plot_at(h, 0) ? c.iplot : 0;
+        p.fstat = fields ? h->d_fstat : nullptr;
+        p.defer = 1;
+        p.part0 = h->d_partials;
+        p.part_stride = (int)h->partials_n;
+        p.partials = h->d_partials + (size_t)(2 + (s & 1)) * h->partials_n;
+        p.prev_partials = h->d_partials + (size_t)(2 + ((s + 1) & 1)) * h->partials_n;
+        return p;
+    };
+    for (int s = 0; s < n;) {
+        int rc;
+        if (h->pairs) {
+            StepParams<T> p[2] = {params(s), params(s + 1)};
+            rc = launch_pair_params<T>(h, cur, p, st);
+            s += 2;
+        } else {
+            StepParams<T> p = params(s);
+            p.src = (const T*)h->buf[cur];
+            p.dst = (T*)h->buf[1 - cur];
+            if constexpr (sizeof(T) == 8) rc = launch_step_f64(p, h->tile_cfg, st, 0);
+            else rc = launch_step_f32(p, h->tile_cfg, st, 0);
+            ++s;
+        }
+        if (rc != 0) return rc;
+        cur ^= 1;
+    }
+    return 0;
+}
+
+// The graph of n steps from the handle's current level (captured on the handle's own stream if none is kept).
+int replay_graph(mrlbm_handle* h, int n, bool fields, mrlbm_handle::Replay*& out) {
+    const bool fp64 = h->precision == MRLBM_FP64;
+    const std::vector<uintptr_t> sig = {(uintptr_t)h->cur, (uintptr_t)h->tile_cfg, (uintptr_t)h->pairs, (uintptr_t)h->mid,
+                                        h->has_uin ? (uintptr_t)h->d_uin : 0, h->has_body ? (uintptr_t)h->d_body : 0,
+                                        fields ? (uintptr_t)h->d_fstat : 0};
+    mrlbm_handle::Replay* g = &h->replay[0];
+    for (auto& q : h->replay) {
+        if (q.exec && q.steps == n && q.sig == sig) {
+            q.used = ++h->replay_clock;
+            out = &q;
+            return MRLBM_OK;
+        }
+        if (q.used < g->used) g = &q;                              // least recently used
+    }
+    if (!h->d_call) CK(cudaMalloc((void**)&h->d_call, 5 * sizeof(int)));
+    if (g->exec) {
+        CK(cudaStreamSynchronize(h->stream));
+        cudaGraphExecDestroy(g->exec);
+        *g = mrlbm_handle::Replay{};
+    }
+    CK(cudaStreamBeginCapture(h->own_stream, cudaStreamCaptureModeThreadLocal));
+    const int rc = fp64 ? capture_run<double>(h, n, fields, h->own_stream) : capture_run<float>(h, n, fields, h->own_stream);
+    cudaGraph_t graph = nullptr;
+    cudaError_t e = cudaStreamEndCapture(h->own_stream, &graph);
+    if (rc == 0 && e == cudaSuccess) e = cudaGraphInstantiate(&g->exec, graph, 0);
+    if (graph) cudaGraphDestroy(graph);
+    if (rc != 0 || e != cudaSuccess) {
+        cudaGetLastError();
+        g->exec = nullptr;
+        if (rc == -2) return fail(h, MRLBM_EUNSUPPORTED, "tile shape does not fit this precision");
+        return fail(h, MRLBM_ECUDA, "capturing a run of steps failed");
+    }
+    g->steps = n;
+    g->sig = sig;
+    g->launches = h->pairs ? n / 2 * PAIR_LAUNCHES : n * step_launches(!fp64, h->tile_cfg);
+    g->used = ++h->replay_clock;
+    out = g;
+    return MRLBM_OK;
+}
+
+int step_replay(mrlbm_handle* h, int n) {
+    const int z = h->iter + n;
+    const bool fields = fields_at(h, h->iter + 1);
+    mrlbm_handle::Replay* g = nullptr;
+    const int rc = replay_graph(h, n, fields, g);
+    if (rc != MRLBM_OK) return rc;
+    // (pageable memory: the copy takes the words before it returns)
+    const int call[5] = {h->iter, h->ring_n, h->pend.on ? h->pend.iter : 0, h->pend.on ? h->pend.rec_idx : -1,
+                         h->pend.on ? h->pend.slot : 0};
+    CK(cudaMemcpyAsync(h->d_call, call, sizeof call, cudaMemcpyHostToDevice, h->stream));
+    CK(cudaGraphLaunch(g->exec, h->stream));
+    h->launches += g->launches;
+    const int lo = std::max(h->iter + 1, h->cfg.statsbegin), hi = std::min(z, h->cfg.statsend);
+    if (h->cfg.post_process && hi >= lo) h->ring_n += hi - lo + 1;
+    h->pend.on = stats_at(h, z);
+    if (h->pend.on) h->pend = mrlbm_handle::Pending{true, 2 + ((n - 1) & 1), h->ring_n - 1, z};
+    if (fields) h->fstat_n += n;
+    h->iter = z;
+    h->cur ^= (h->pairs ? n / 2 : n) & 1;
+    return MRLBM_OK;
+}
+
 void free_all(mrlbm_handle* h) {
     if (h->host_only) return;
     cudaSetDevice(h->device);
+    for (auto& q : h->replay)
+        if (q.exec) cudaGraphExecDestroy(q.exec);
     for (void* p : {h->buf[0], h->buf[1], h->mid, h->d_bgeo, (void*)h->d_bint, (void*)h->d_boxmap, (void*)h->d_partials,
                     (void*)h->d_counter, (void*)h->d_ring, (void*)h->d_err, (void*)h->d_macro, (void*)h->d_uin, h->d_body, (void*)h->d_ovr, h->adj_ws, (void*)h->d_fstage,
-                    (void*)h->d_tile_ctr, (void*)h->d_fstat, (void*)h->d_fstat_out, (void*)h->d_quad, (void*)h->d_W,
+                    (void*)h->d_tile_ctr, (void*)h->d_call, (void*)h->d_fstat, (void*)h->d_fstat_out, (void*)h->d_quad, (void*)h->d_W,
                     (void*)h->d_sumw, (void*)h->d_sring, (void*)h->d_pring, (void*)h->d_sidx})
         if (p) cudaFree(p);
     if (h->h_ring) cudaFreeHost(h->h_ring);
@@ -813,7 +983,7 @@ static int create_impl(const mrlbm_config* cfg, int precision, int device, int s
     ok = ok && ck(cudaMalloc((void**)&h->d_boxmap, nbox * sizeof(int)), "cudaMalloc boxmap");
     const size_t nscratch = 2 * (size_t)nb + (size_t)ny + 8;
     h->partials_n = nscratch;
-    ok = ok && ck(cudaMalloc((void**)&h->d_partials, 2 * nscratch * sizeof(double)), "cudaMalloc partials") &&
+    ok = ok && ck(cudaMalloc((void**)&h->d_partials, 4 * nscratch * sizeof(double)), "cudaMalloc partials") &&
          ck(cudaMalloc((void**)&h->d_counter, 3 * sizeof(unsigned)), "cudaMalloc counter") &&
          ck(cudaMalloc((void**)&h->d_ring, (size_t)RING_CAP * REC_WORDS * sizeof(double)), "cudaMalloc ring") &&
          ck(cudaMalloc((void**)&h->d_err, sizeof(int)), "cudaMalloc err") &&
@@ -1313,7 +1483,13 @@ int mrlbm_step(mrlbm_handle* h, int32_t nsteps, int32_t flags) {
     for (int s = 0; s < nsteps;) {
         int rc;
         // a step with macroscopic output is taken alone
-        if (nsteps - s >= ((flags & MRLBM_STEP_MACRO) ? 3 : 2) && pair_ok(h)) {
+        const int s0 = s;
+        const int run = replay_length(h, nsteps - s - ((flags & MRLBM_STEP_MACRO) ? 1 : 0));
+        if (run > 0) {
+            rc = step_replay(h, run);
+            if (rc != MRLBM_OK) return rc;
+            s += run;
+        } else if (nsteps - s >= ((flags & MRLBM_STEP_MACRO) ? 3 : 2) && pair_ok(h)) {
             rc = launch_two(h);
             if (rc != MRLBM_OK) return rc;
             s += 2;
@@ -1327,6 +1503,7 @@ int mrlbm_step(mrlbm_handle* h, int32_t nsteps, int32_t flags) {
             }
             ++s;
         }
+        h->stepped += s - s0;
         if (h->ring_n == RING_CAP) {
             rc = drain_ring(h);
             if (rc != MRLBM_OK) return rc;
@@ -1514,6 +1691,7 @@ int mrlbm_autotune(mrlbm_handle* h, int32_t trial_steps, int32_t* best_cfg, doub
     int rc = MRLBM_OK;
     // every shape by single steps, then (index N_ALL_CFGS) the best of them with its steps in pairs
     const bool pairs0 = h->pairs;
+    h->no_replay = true;
     const int last = h->pairs_fixed || std::min(h->L.nx, h->L.ny) < 64 ? N_ALL_CFGS : N_ALL_CFGS + 1;
     bool pairs_best = false;
     for (int c = 0; c < last && rc == MRLBM_OK; ++c) {
@@ -1567,6 +1745,7 @@ int mrlbm_autotune(mrlbm_handle* h, int32_t trial_steps, int32_t* best_cfg, doub
     cudaEventDestroy(e1);
     cudaStreamSynchronize(h->stream);
     cleanup();
+    h->no_replay = false;
     if (rc != MRLBM_OK) {
         h->tile_cfg = cfg0;
         h->pairs = pairs0;

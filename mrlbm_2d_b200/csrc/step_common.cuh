@@ -309,6 +309,28 @@ __device__ __forceinline__ StepRec step_rec(const StepParams<T>& p) {
     return r;
 }
 
+// The deferred record this step has to sum (StepParams::defer): the launch's own, or for a replayed
+// launch the step before it, if that was a stats step.  False when there is none.
+template <class T>
+__device__ __forceinline__ bool prev_record(const StepParams<T>& p, const double*& part, double*& rec, int& iter) {
+    part = p.prev_partials;
+    rec = p.prev_rec;
+    iter = p.prev_iter;
+    if (!p.call) return rec != nullptr;
+    if (p.bstep == 0) {
+        const int idx = __ldg(p.call + 3);
+        iter = __ldg(p.call + 2);
+        part = p.part0 + (size_t)__ldg(p.call + 4) * p.part_stride;
+        rec = p.ring + (size_t)max(idx, 0) * REC_WORDS;
+        return idx >= 0;
+    }
+    const int iter0 = __ldg(p.call), rn0 = __ldg(p.call + 1);
+    iter = iter0 + p.bstep;
+    const int before = max(0, min(iter - 1, p.stats_hi) - max(iter0 + 1, p.stats_lo) + 1);
+    rec = p.ring + (size_t)(rn0 + before) * REC_WORDS;
+    return iter >= p.stats_lo && iter <= p.stats_hi;
+}
+
 // Force tail, called by every boundary block once its nodes' forces are in p.partials.
 template <class Phys>
 __device__ __forceinline__ void force_tail(const typename Phys::P& p, const StepRec& sr, unsigned char* smem) {
@@ -470,10 +492,13 @@ __device__ __forceinline__ void boundary_block(const typename Phys::P& p, unsign
 template <class Phys>
 __device__ __forceinline__ void edge_block(const typename Phys::P& p, int eb, unsigned char* smem) {
     const int nx = p.L.nx, ny = p.L.ny;
-    if (p.defer && p.prev_rec && eb == p.neblk - 1) {
+    if (p.defer && (p.prev_rec || p.call) && eb == p.neblk - 1) {
         // a block of its own for the in-order sums: behind an edge node's chain they made the last edge
         // block of a 400 x 100 step take 4.7 us where the others took 1.6
-        record_sums(p.prev_partials, p.nb, ny, p.halo_l, p.prev_rec, p.prev_iter, smem);
+        const double* part;
+        double* rec;
+        int iter;
+        if (prev_record(p, part, rec, iter)) record_sums(part, p.nb, ny, p.halo_l, rec, iter, smem);
         return;
     }
     const StepRec sr = step_rec(p);
@@ -564,7 +589,7 @@ __device__ __forceinline__ void bulk_end(const StepParams<T>& p) {
 
 template <class P>
 inline int edge_blocks(const P& p, int nthr) {
-    return (edge_threads(p.L.nx, p.L.ny, p.halo_l, p.halo_r) + nthr - 1) / nthr + (p.defer && p.prev_rec ? 1 : 0);
+    return (edge_threads(p.L.nx, p.L.ny, p.halo_l, p.halo_r) + nthr - 1) / nthr + (p.defer && (p.prev_rec || p.call) ? 1 : 0);
 }
 
 template <class Phys>

@@ -81,12 +81,17 @@ struct alignas(64) StepParams {
     const double* prev_partials;  // terms of the last stats step still to be summed, or null
     double* prev_rec;             // its record
     int prev_iter;
+    // the handle's partials slots (a replayed first step finds its predecessor's by the call state)
+    const double* part0;
+    int part_stride;
     double* node_force;           // optional per-boundary-node (Fx, Fy) [2 * nb], or null
     int iter;
     // A launch captured once into a replayed graph (a batch's per-case streams schedule): `call`
     // points at the state {iter0, ring_n0} uploaded before each replay, and the record fields
     // (iter, do_stats, rec) come from it instead (step_rec): iteration iter0 + bstep + 1, a
     // record when it lies in [stats_lo, stats_hi], in `ring` after the call's earlier records.
+    // With deferred sums (a single case's replayed steps) three more words tell which record was
+    // still to be summed when the call began: {iteration, ring index or -1, partials slot}.
     const int* call;
     int bstep, stats_lo, stats_hi;
     double* ring;
