@@ -2049,7 +2049,7 @@ int stats_in(const mrlbm_config& c, int a, int z) {
 void batch_items(const mrlbm_handle* h, int cfg, int aux_threads, int& aux, int& tiles, int& nbblk, int& neblk,
                  int& tiles_x) {
     nbblk = wall_blocks(h->geo.nb, aux_threads, h->precision == MRLBM_FP64);
-    neblk = (edge_threads(h->L.nx, h->L.ny, h->halo_l, h->halo_r) + aux_threads - 1) / aux_threads;
+    neblk = edge_split(h->L.nx, h->L.ny, h->halo_l, h->halo_r, aux_threads).blocks;
     int tiles_y;
     if (is_vec_cfg(cfg)) {
         const VecCfg v = VEC_CFGS[cfg - VEC_CFG0];

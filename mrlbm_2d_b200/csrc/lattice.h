@@ -77,12 +77,21 @@ MRLBM_HD SrcSlot stream_source(int nx, int ny, int i, int j, int k, bool xper, b
     return s;
 }
 
-// Threads of the edge blocks' enumeration (edge_block, step_common.cuh): column 1, column nx, row 1 and row
-// ny without the corners, each group rounded up to whole warps so that no warp mixes two kinds of
-// edge.  An x-slab's halo faces are not edges.
-MRLBM_HD int edge_pad(int n) { return (n + 31) & ~31; }
-MRLBM_HD int edge_threads(int nx, int ny, bool hl, bool hr) {
-    return (hl ? 0 : edge_pad(ny)) + (hr ? 0 : edge_pad(ny)) + 2 * edge_pad(nx - (hl ? 0 : 1) - (hr ? 0 : 1));
+// Edge blocks (edge_block, step_common.cuh).  The edge nodes are split into warps of one kind: column 1, column
+// nx, row 1, row ny without the corners; an x-slab's halo faces are not edges.  A column's nodes lie a
+// row apart, so each of a warp's loads and stores is 32 separate sectors, and eight such warps on one SM
+// took 2.4 us for their requests alone: the column warps are dealt to blocks of their own first, the
+// row warps fill up behind them.
+MRLBM_HD int edge_warps(int n) { return (n + 31) >> 5; }
+struct EdgeSplit { int left, right, row, blocks; };       // warps of column 1, of column nx, of one row; blocks
+MRLBM_HD EdgeSplit edge_split(int nx, int ny, bool hl, bool hr, int threads) {
+    EdgeSplit s;
+    s.left = hl ? 0 : edge_warps(ny);
+    s.right = hr ? 0 : edge_warps(ny);
+    s.row = edge_warps(nx - (hl ? 0 : 1) - (hr ? 0 : 1));
+    const int per = threads >> 5, all = (s.left + s.right + 2 * s.row + per - 1) / per, col = s.left + s.right;
+    s.blocks = all > col ? all : col;
+    return s;
 }
 
 // Node class inside the cylinder bounding box (values >= 0 are boundary-node indices).

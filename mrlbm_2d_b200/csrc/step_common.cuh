@@ -370,10 +370,8 @@ __device__ __forceinline__ void record_sums(const double* part, int nb, int ny, 
     if (tid == 0) rec[0] = (double)iter;
 }
 
-// Edge blocks [0, inlet_blocks) hold the inlet column (it comes first in their enumeration).
-__device__ __forceinline__ int inlet_blocks(int ny, int halo_l) {
-    return halo_l ? 0 : (ny + (int)blockDim.x - 1) / (int)blockDim.x;
-}
+// Edge blocks [0, inlet_blocks) hold the inlet column (a warp each, edge_split).
+__device__ __forceinline__ int inlet_blocks(int ny, int halo_l) { return halo_l ? 0 : edge_warps(ny); }
 
 // Inlet tail, called by every edge block once its inlet nodes' rho are in p.partials.
 template <class Phys>
@@ -484,10 +482,9 @@ __device__ __forceinline__ void boundary_block(const typename Phys::P& p, unsign
     if (!p.defer) force_tail<Phys>(p, sr, smem);
 }
 
-// Edge blocks: one thread per domain-edge node, so the edge closures (outlet neighbour gather,
-// inlet/outlet/wall closures, 2d_mrlbm.f90:249-272, 313-351) run side by side instead of
-// serially inside bulk tiles.  Order: column 1 (j = 1..ny), column nx, then rows 1 and ny
-// without the corners; an x-slab's halo faces are not edges.  The thread of node (1,j) also
+// Edge blocks: one thread per domain-edge node (edge_split), so the edge closures (outlet neighbour
+// gather, inlet/outlet/wall closures, 2d_mrlbm.f90:249-272, 313-351) run side by side instead of
+// serially inside bulk tiles.  The thread of node (1,j) also
 // records rho(1,j) after the closures for the inlet running mean (2d_mrlbm.f90:359).
 template <class Phys>
 __device__ __forceinline__ void edge_block(const typename Phys::P& p, int eb, unsigned char* smem) {
@@ -502,20 +499,20 @@ __device__ __forceinline__ void edge_block(const typename Phys::P& p, int eb, un
         return;
     }
     const StepRec sr = step_rec(p);
-    const int e = eb * (int)blockDim.x + (int)threadIdx.x;
-    const int cl = p.halo_l ? 0 : 1, cr = p.halo_r ? 0 : 1;         // edge columns of this lattice
-    const int nl = cl * edge_pad(ny), nr = cr * edge_pad(ny), nrow = nx - cl - cr, rp = edge_pad(nrow);
+    const EdgeSplit es = edge_split(nx, ny, p.halo_l, p.halo_r, (int)blockDim.x);
+    const int lane = (int)threadIdx.x & 31, t = (int)(threadIdx.x >> 5) * es.blocks + eb;   // this warp's place in the split
+    const int cl = p.halo_l ? 0 : 1, nrow = nx - cl - (p.halo_r ? 0 : 1);
     int i, j;
     bool on;
-    if (e < nl + nr) {
-        i = e < nl ? 1 : nx;
-        j = 1 + (e < nl ? e : e - nl);
+    if (t < es.left + es.right) {
+        i = t < es.left ? 1 : nx;
+        j = 1 + 32 * (t < es.left ? t : t - es.left) + lane;
         on = j <= ny;
     } else {
-        const int q = e - nl - nr, side = q >= rp;
-        i = cl + 1 + (q - side * rp);
+        const int q = t - es.left - es.right, side = q >= es.row, at = 32 * (q - side * es.row) + lane;
+        i = cl + 1 + at;
         j = side ? ny : 1;
-        on = q < 2 * rp && i <= cl + nrow;
+        on = q < 2 * es.row && at < nrow;
     }
     if (on) {
         const double rho = Phys::edge_bulk_node(p, i, j, CLS_FLUID);
@@ -589,7 +586,7 @@ __device__ __forceinline__ void bulk_end(const StepParams<T>& p) {
 
 template <class P>
 inline int edge_blocks(const P& p, int nthr) {
-    return (edge_threads(p.L.nx, p.L.ny, p.halo_l, p.halo_r) + nthr - 1) / nthr + (p.defer && (p.prev_rec || p.call) ? 1 : 0);
+    return edge_split(p.L.nx, p.L.ny, p.halo_l, p.halo_r, nthr).blocks + (p.defer && (p.prev_rec || p.call) ? 1 : 0);
 }
 
 template <class Phys>
