@@ -1411,13 +1411,15 @@ int mrlbm_surface_enable(mrlbm_handle* h, int32_t enable) {
         CK(cudaMalloc((void**)&h->d_sring, (size_t)h->surf_cap * 2 * nb * sizeof(double)));
         CK(cudaMalloc((void**)&h->d_pring, (size_t)h->surf_cap * 12 * sizeof(double)));
         CK(cudaMemcpyAsync(h->d_quad, quad.data(), quad.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-        CK(cudaMemcpyAsync(h->d_sidx, idx.data(), nb * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+        std::vector<int> place(nb);
+        for (int i = 0; i < nb; ++i) place[idx[i]] = i;
+        CK(cudaMemcpyAsync(h->d_sidx, place.data(), nb * sizeof(int), cudaMemcpyHostToDevice, h->stream));
         CK(cudaMemcpyAsync(h->d_W, W.data(), W.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
         CK(cudaMemcpyAsync(h->d_sumw, sumw.data(), nb * sizeof(double), cudaMemcpyHostToDevice, h->stream));
         CK(cudaStreamSynchronize(h->stream));
     }
     h->surf.quad = h->d_quad;
-    h->surf.idx = h->d_sidx;
+    h->surf.place = h->d_sidx;
     h->surf.W = h->d_W;
     h->surf.sumw = h->d_sumw;
     h->surf.nb = nb;

@@ -8,7 +8,7 @@ namespace mrlbm {
 // Per-case constant tables of the surface output.
 struct SurfaceTables {
     const double* quad;     // [5 * nb] per wall node: r(point 2), r(point 3), r(point 4), r(point 1), denom
-    const int* idx;         // [nb] wall-node order by increasing theta (2d_mrlbm.f90:1138-1156)
+    const int* place;       // position of wall node l in theta order
     const double* W;        // [nb * nb] Gaussian weights, W[j * nb + i] (column j contiguous over i)
     const double* sumw;     // [nb] sum_j W[j * nb + i] in index order
     int probe_i[4], probe_j[4];
