@@ -360,7 +360,8 @@ int mrlbm_slabs_step(mrlbm_handle** hs, int32_t n, int32_t nsteps);
  * case's own, steps_per_launch steps per case captured into one graph and replayed with the
  * per-call iteration and record slots uploaded before each replay (MRLBM_BATCH_STREAMS; a call
  * with macroscopic output, field statistics or a loaded state's first step runs as
- * MRLBM_BATCH_GRAPH instead).  Each case's results are bit-identical to stepping it alone.  The
+ * MRLBM_BATCH_GRAPH instead; the autotuner may choose it with the steps taken in pairs, see
+ * mrlbm_step).  Each case's results are bit-identical to stepping it alone.  The
  * cases are ordinary handles owned by the batch (mrlbm_batch_case): read their forces,
  * fields and state, load states, set inlet profiles and field-statistics windows with the
  * single-case calls, but step them only through mrlbm_batch_step and do not destroy them.

@@ -526,7 +526,7 @@ bool pairs_pay(const mrlbm_handle* h) {
 }
 
 // Nodes the two-step tiles leave out and the band of the intermediate level (PairPlan).
-void make_pair_plan(mrlbm_handle* h) {
+void make_pair_plan(mrlbm_handle* h, int sharers) {
     const Geometry& g = h->geo;
     PairPlan& q = h->plan;
     q.core = q.halo = PairRect{1, 0, 1, 0};
@@ -542,12 +542,13 @@ void make_pair_plan(mrlbm_handle* h) {
                 q.halo.y1 = std::max(q.halo.y1, j + 1);
             }
     }
-    q.chunks = pair_chunks(h->L.nx, h->L.ny, h->elem == 8 ? PAIR_STRIPS64 : PAIR_STRIPS32, PAIR_MINB * h->num_sms);
+    q.chunks = pair_chunks(h->L.nx, h->L.ny, h->elem == 8 ? PAIR_STRIPS64 : PAIR_STRIPS32, std::max(1, PAIR_MINB * h->num_sms / sharers));
 }
 
+// `sharers`: cases that step on the GPU at the same time (a batch), each with its part of the resident blocks.
 // Take steps in pairs from now on: the band buffer, with the ghost ring every level carries.
 // False (and single steps as before) when there is no memory for it.
-bool enable_pairs(mrlbm_handle* h) {
+bool enable_pairs(mrlbm_handle* h, int sharers = 1) {
     if (!pairs_possible(h)) return false;
     if (!h->mid) {
         auto enc = tensor_map_encoder();
@@ -567,8 +568,8 @@ bool enable_pairs(mrlbm_handle* h) {
             return false;
         }
         if (launch_copy_ring(h->precision, h->buf[h->cur], h->mid, h->L, h->stream) != cudaSuccess) return false;
-        make_pair_plan(h);
     }
+    make_pair_plan(h, sharers);
     h->pairs = true;
     return true;
 }
@@ -2021,9 +2022,13 @@ struct mrlbm_batch {
     struct StreamsGraph {
         cudaGraphExec_t exec = nullptr;
         int cfg = -1, steps = 0;
-        std::vector<uintptr_t> sig;    // per case: time level, inlet-profile and body-force buffers when captured
+        bool pairs = false;
+        std::vector<uintptr_t> sig;    // per case: time level, inlet-profile, body-force and band buffers when captured
     } sg[2];
     int sg_next = 0;
+    // the autotuner's choice: per-case streams whose steps are taken in pairs (step_pair.cuh); every case then
+    // has its band buffer
+    bool pairs = false, pairs_fixed = false;   // fixed: by MRLBM_PAIRS at creation
 };
 
 namespace {
@@ -2157,12 +2162,21 @@ int streams_launch_case(mrlbm_batch* b, int c, int steps) {
     p.ring = h->d_ring;
     p.plot_every = k.post_process && k.iplot > 0 && (k.channel_with_cylinder || k.channel_with_square) ? k.iplot : 0;
     int cur = h->cur;
-    for (int s = 0; s < steps; ++s) {
-        p.src = (const T*)h->buf[cur];
-        p.dst = (T*)h->buf[1 - cur];
+    for (int s = 0; s < steps;) {
+        int rc;
         p.bstep = s;
-        const int rc = sizeof(T) == 8 ? launch_step_f64(reinterpret_cast<const StepParams<double>&>(p), b->tile_cfg, b->cstream[c], 0)
-                                      : launch_step_f32(reinterpret_cast<const StepParams<float>&>(p), b->tile_cfg, b->cstream[c], 0);
+        if (b->pairs && s + 1 < steps) {
+            StepParams<T> q[2] = {p, p};
+            q[1].bstep = s + 1;
+            rc = launch_pair_params<T>(h, cur, q, b->cstream[c]);
+            s += 2;
+        } else {
+            p.src = (const T*)h->buf[cur];
+            p.dst = (T*)h->buf[1 - cur];
+            rc = sizeof(T) == 8 ? launch_step_f64(reinterpret_cast<const StepParams<double>&>(p), b->tile_cfg, b->cstream[c], 0)
+                                : launch_step_f32(reinterpret_cast<const StepParams<float>&>(p), b->tile_cfg, b->cstream[c], 0);
+            ++s;
+        }
         if (rc != 0) return rc;
         cur ^= 1;
     }
@@ -2200,16 +2214,17 @@ int batch_call_streams(mrlbm_batch* b, int steps) {
     BCK(cudaEventRecord(b->call_staged, b->stream));
     // the graph captured for these cases' time levels (two are kept: an odd call length
     // alternates them)
-    std::vector<uintptr_t> sig(3 * (size_t)n);
+    std::vector<uintptr_t> sig(4 * (size_t)n);
     for (int c = 0; c < n; ++c) {
         const mrlbm_handle* h = b->h[c];
-        sig[3 * c] = (uintptr_t)h->cur;
-        sig[3 * c + 1] = h->has_uin ? (uintptr_t)h->d_uin : 0;
-        sig[3 * c + 2] = h->has_body ? (uintptr_t)h->d_body : 0;
+        sig[4 * c] = (uintptr_t)h->cur;
+        sig[4 * c + 1] = h->has_uin ? (uintptr_t)h->d_uin : 0;
+        sig[4 * c + 2] = h->has_body ? (uintptr_t)h->d_body : 0;
+        sig[4 * c + 3] = b->pairs ? (uintptr_t)h->mid : 0;
     }
     mrlbm_batch::StreamsGraph* g = nullptr;
     for (auto& q : b->sg)
-        if (q.exec && q.cfg == b->tile_cfg && q.steps == steps && q.sig == sig) g = &q;
+        if (q.exec && q.cfg == b->tile_cfg && q.steps == steps && q.pairs == b->pairs && q.sig == sig) g = &q;
     if (!g) {
         g = &b->sg[b->sg_next];
         b->sg_next ^= 1;
@@ -2238,14 +2253,16 @@ int batch_call_streams(mrlbm_batch* b, int steps) {
         if (e != cudaSuccess) return bfail(b, MRLBM_ECUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
         g->cfg = b->tile_cfg;
         g->steps = steps;
+        g->pairs = b->pairs;
         g->sig = sig;
     }
     BCK(cudaGraphLaunch(g->exec, b->stream));
+    const int pairs = b->pairs ? steps / 2 : 0, singles = steps - 2 * pairs;
     for (mrlbm_handle* h : b->h) {
         h->ring_n += stats_in(h->cfg, h->iter + 1, h->iter + steps);
         h->iter += steps;
-        h->cur ^= steps & 1;
-        b->launches += (int64_t)steps * step_launches(!fp64, b->tile_cfg);
+        h->cur ^= (pairs + singles) & 1;
+        b->launches += (int64_t)pairs * PAIR_LAUNCHES + (int64_t)singles * step_launches(!fp64, b->tile_cfg);
     }
     return MRLBM_OK;
 }
@@ -2450,8 +2467,13 @@ int mrlbm_batch_create(const mrlbm_config* cfgs, int32_t ncases, int precision, 
             h->own_stream = nullptr;
         }
         h->stream = b->stream;
-        disable_pairs(h);                              // a batch steps its cases one step at a time
+        b->pairs_fixed = b->pairs_fixed || h->pairs_fixed;
+        b->pairs = (c == 0 || b->pairs) && h->pairs && h->pairs_fixed;
     }
+    if (b->pairs)
+        for (mrlbm_handle* h : b->h) enable_pairs(h, ncases);
+    else
+        for (mrlbm_handle* h : b->h) disable_pairs(h);  // one step at a time until the autotuner finds otherwise
     b->stage_bytes = batch_param_bytes(b);
     bool ok = cudaMalloc(&b->d_params, b->stage_bytes) == cudaSuccess &&
               cudaMalloc((void**)&b->d_cases, sizeof(BatchCase) * ncases) == cudaSuccess &&
@@ -2497,6 +2519,7 @@ int mrlbm_batch_set_schedule(mrlbm_batch* b, int32_t tile_cfg, int32_t schedule,
     b->tile_cfg = tile_cfg;
     b->schedule = schedule;
     b->steps_per_launch = steps_per_launch;
+    if (!b->pairs_fixed) b->pairs = false;
     return MRLBM_OK;
 }
 
@@ -2604,11 +2627,14 @@ int mrlbm_batch_autotune(mrlbm_batch* b, int32_t trial_steps, double* best_ms_pe
     };
     const int tile0 = b->tile_cfg, sched0 = b->schedule, spl0 = b->steps_per_launch;
     int best_tile = tile0, best_sched = sched0, best_spl = spl0;
-    double best = 1e300;
+    double best = 1e300, best_streams = 1e300;
+    int streams_tile = -1;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     const int steps = std::min((trial_steps + 1) & ~1, RING_CAP);   // even: a call ends on its start level
+    const bool pairs0 = b->pairs;
+    if (!b->pairs_fixed) b->pairs = false;
     for (int cfg = 0; cfg < PIPE_CFG0 && rc == MRLBM_OK; ++cfg) {
         if (cfg >= N_TILE_CFGS && cfg < VEC_CFG0) continue;     // TMA shapes are single-case only
         for (int sched = MRLBM_BATCH_PERSISTENT; sched <= MRLBM_BATCH_STREAMS && rc == MRLBM_OK; ++sched) {
@@ -2627,7 +2653,35 @@ int mrlbm_batch_autotune(mrlbm_batch* b, int32_t trial_steps, double* best_ms_pe
             float ms = 0.f;
             cudaEventElapsedTime(&ms, e0, e1);
             if (ms < best) { best = ms; best_tile = cfg; best_sched = sched; best_spl = steps; }
+            if (sched == MRLBM_BATCH_STREAMS && ms < best_streams) { best_streams = ms; streams_tile = cfg; }
             restore();
+        }
+    }
+    // per-case streams with the steps in pairs, if every case can take them and has the memory
+    bool pairs_best = pairs0 && b->pairs_fixed;
+    bool able = rc == MRLBM_OK && streams_tile >= 0 && steps <= STREAMS_MAX_STEPS && !b->pairs_fixed;
+    for (size_t c = 0; c < b->h.size() && able; ++c) able = enable_pairs(b->h[c], (int)b->h.size());
+    if (able) {
+        b->tile_cfg = streams_tile;
+        b->schedule = MRLBM_BATCH_STREAMS;
+        b->steps_per_launch = steps;
+        b->pairs = true;
+        // warm-up from either time level (an odd number of pairs changes it) and past a loaded state's first step
+        for (int w = 0; w < 3 && rc == MRLBM_OK; ++w) rc = batch_call(b, steps, 0);
+        if (rc == MRLBM_OK) {
+            cudaEventRecord(e0, b->stream);
+            rc = batch_call(b, steps, 0);
+            cudaEventRecord(e1, b->stream);
+            if (rc == MRLBM_OK && cudaEventSynchronize(e1) != cudaSuccess) rc = MRLBM_ECUDA;
+            float ms = 0.f;
+            if (rc == MRLBM_OK) cudaEventElapsedTime(&ms, e0, e1);
+            if (rc == MRLBM_OK && ms < best) {
+                best = ms;
+                best_tile = streams_tile;
+                best_sched = MRLBM_BATCH_STREAMS;
+                best_spl = steps;
+                pairs_best = true;
+            }
         }
     }
     restore();
@@ -2638,6 +2692,9 @@ int mrlbm_batch_autotune(mrlbm_batch* b, int32_t trial_steps, double* best_ms_pe
         for (void* q : s.buf) if (q) cudaFree(q);
         if (s.fstat) cudaFree(s.fstat);
     }
+    b->pairs = rc == MRLBM_OK ? pairs_best : pairs0;
+    if (!b->pairs)
+        for (mrlbm_handle* h : b->h) disable_pairs(h);
     if (rc != MRLBM_OK) {
         b->tile_cfg = tile0; b->schedule = sched0; b->steps_per_launch = spl0;
         return rc;

@@ -124,3 +124,27 @@ def test_pairs_over_a_long_run_of_full_waves(mrlbm, monkeypatch, prec):
     assert np.array_equal(res[0][0], res[1][0])
     for x, y in zip(res[0][1], res[1][1]):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("prec", [64, 32])
+def test_batch_streams_in_pairs(mrlbm, monkeypatch, prec):
+    """Per-case streams with the steps in pairs, odd and even call lengths, against each case alone."""
+    cfgs = [CASES[n]() for n in ("freeslip_label15", "reference_default_bcs", "reference_walls")]
+    cfgs.append(cylinder_case(256, 64, 12.8, 51.2, 32.5, 150.0, 0.05))
+    monkeypatch.setenv("MRLBM_PAIRS", "1")
+    b = mrlbm.Batch(cfgs, precision=prec)
+    b.set_schedule(9, mrlbm.BATCH_STREAMS, 6)
+    for n in (6, 12, 9, 5):                         # whole graphs, both start levels, remainders
+        b.step(n)
+    b.step(7, macro=True)
+    assert b.status() == 0
+    monkeypatch.setenv("MRLBM_PAIRS", "0")
+    for cfg, c in zip(cfgs, b.cases):
+        s = mrlbm.Simulation(cfg, precision=prec)
+        s.step(39, macro=True)
+        assert np.array_equal(c.get_state(), s.get_state())
+        for x, y in zip(c.forces(), s.forces()):
+            assert np.array_equal(x, y)
+        assert np.array_equal(c.macro()["ux"], s.macro()["ux"])
+        s.close()
+    b.close()
