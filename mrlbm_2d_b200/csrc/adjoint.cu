@@ -10,7 +10,7 @@ namespace mrlbm {
 template <class T>
 static int launch_adjoint(const StepParams<T>& p, const adj::AdjArgs& a, cudaStream_t s) {
     const int64_t nodes = (int64_t)p.L.nx * p.L.ny;
-    const int64_t aux = (int64_t)p.nb + (a.n_edge + 6) / 7;
+    const int64_t aux = (int64_t)adj::adjoint_wall_blocks(p.closure, p.nb) + (a.n_edge + 6) / 7;
     cudaError_t e;
     switch (p.closure) {                               // the curved-wall closure, one instantiation each
     case CLOSURE_STRONG: e = launch_after_prior(adj::adjoint_aux<StepParams<T>, CLOSURE_STRONG>, (unsigned)aux, 128, 0, s, p, a); break;

@@ -18,8 +18,9 @@
 //     local map evaluated on dual numbers carrying the derivative along that input, then
 //     contracted with lambda^n (the transposed Jacobian column); the inlet's extra input is
 //     u_in(j), whose column gives the inlet-profile gradient;
-//   * curved-wall nodes: likewise, over the node's 9 own inputs and the 72 inputs of its 8
-//     bilinear stencil nodes, with the drag contribution of the node in the same pass.
+//   * curved-wall nodes, their drag contribution in the same pass: reverse mode by hand (adjoint_wall);
+//     with the unrotated closure on dual numbers like the edge nodes, over the node's 9 own inputs and
+//     the 72 inputs of its 8 bilinear stencil nodes.
 // The local maps below restate the FP64 step's arithmetic (step_fp64.cuh) for a generic
 // scalar; they cover every closure of the FP64 step: the curved-wall closures (rotated
 // strong, weak and rho_eq, unrotated with Cramer's rule, none) with or without velocity and
@@ -43,6 +44,14 @@ template <class T>
 __device__ __forceinline__ void gather_d(const StepParams<T>& p, int i, int j, double f[Q]) {
     T g[Q];
     gather(p, i, j, g);
+#pragma unroll
+    for (int k = 0; k < Q; ++k) f[k] = to_f(p, k, g[k]);
+}
+
+template <class T>
+__device__ __forceinline__ void edge_gather_d(const StepParams<T>& p, int i, int j, double f[Q]) {
+    T g[Q];
+    edge_gather(p, i, j, g);
 #pragma unroll
     for (int k = 0; k < Q; ++k) f[k] = to_f(p, k, g[k]);
 }
@@ -250,65 +259,6 @@ __device__ __forceinline__ void stencil_quad(const P& p, int l, int s, const S f
     my = m.mxx * s2q + m.myy * c2 - m.mxy * sn2;
 }
 
-// Rotated closures (2d_mrlbm.f90:1635-1765 strong, 1767-1871 weak, 1873-1972 rho_eq) of wall
-// node l for a generic scalar, as closure_rotated_body in step_fp64.cuh: density and the
-// rotated shear moment from the incoming populations, the extrapolated rotated normal moments
-// Mxx, Myy, then the moments rotated back.
-template <int variant, class P, class S>
-__device__ __forceinline__ void closure_rotated_s(const P& p, int l, const S f[Q], S uxp, S uyp, S Mxx, S Myy, MacS<S>& m) {
-    const int Is = gi(p, I_IS, l), Os = gi(p, I_OS, l);
-    const double omega = p.omega;
-    S rhoI = 0.0, mxyI = 0.0, A_p = 0.0, E_p = 0.0, D_xy = 0.0;
-    double B11 = 0, B22 = 0, B12 = 0, F11 = 0, F22 = 0, F12 = 0;
-#pragma unroll
-    for (int k = 0; k < Q; ++k) {
-        const double cxp = gf(p, G_CXP + k, l), cyp = gf(p, G_CYP + k, l);
-        const double hxx = gf(p, G_HXXP + k, l), hyy = gf(p, G_HYYP + k, l), hxy = gf(p, G_HXYP + k, l);
-        const double wk = p.w[k];
-        const S A_i = wk * (1.0 + 3.0 * uxp * cxp + 3.0 * uyp * cyp);
-        const S E_i = wk * (1.0 + 3.0 * uxp * cxp + 3.0 * uyp * cyp + 4.5 * (uxp * uxp) * hxx + 4.5 * (uyp * uyp) * hyy +
-                            9.0 * (uxp * uyp) * hxy);
-        const double B11_i = 4.5 * wk * hxx, B22_i = 4.5 * wk * hyy, B12_i = 4.5 * wk * hxy;
-        const bool o = (Os >> k) & 1, in = (Is >> k) & 1;
-        if constexpr (variant == CLOSURE_STRONG) if (o) { A_p = A_p + A_i; E_p = E_p + E_i; B11 += B11_i; B22 += B22_i; B12 += B12_i; }
-        if (in) {
-            rhoI = rhoI + f[k];
-            mxyI = mxyI + f[k] * hxy;
-            if constexpr (variant == CLOSURE_WEAK) { A_p = A_p + A_i; B11 += B11_i; B22 += B22_i; B12 += B12_i; }
-            if constexpr (variant == CLOSURE_RHOEQ) E_p = E_p + E_i;
-            D_xy = D_xy + A_i * hxy;
-            F11 += B11_i * hxy;
-            F22 += B22_i * hxy;
-            F12 += B12_i * hxy;
-        }
-    }
-    mxyI = mxyI / rhoI;
-    S Mxy;
-    if constexpr (variant == CLOSURE_STRONG) {
-        const S G_p = (1.0 - omega) * A_p + omega * E_p;
-        const double J11 = (1.0 - omega) * B11, J22 = (1.0 - omega) * B22, J12 = (1.0 - omega) * B12;
-        const S L11 = J11 * mxyI - F11, L22 = J22 * mxyI - F22, L12 = 2.0 * (J12 * mxyI - F12);
-        const S R = D_xy - G_p * mxyI;
-        Mxy = (R - Mxx * L11 - Myy * L22) / L12;
-        const S den = (1.0 - omega) * A_p + (1.0 - omega) * (Mxx * B11 + Myy * B22 + 2.0 * Mxy * B12) + omega * E_p;
-        m.rho = rhoI / den;
-    } else if constexpr (variant == CLOSURE_WEAK) {
-        const S L11 = B11 * mxyI - F11, L22 = B22 * mxyI - F22, L12 = 2.0 * (B12 * mxyI - F12);
-        const S R = D_xy - A_p * mxyI;
-        Mxy = (R - Mxx * L11 - Myy * L22) / L12;
-        const S den = A_p + (Mxx * B11 + Myy * B22 + 2.0 * Mxy * B12);
-        m.rho = rhoI / den;
-    } else {                                               // CLOSURE_RHOEQ
-        const S R = E_p * mxyI - D_xy;
-        Mxy = (R - Mxx * F11 - Myy * F22) / (2.0 * F12);
-        m.rho = rhoI / E_p;
-    }
-    const double cc = gf(p, G_CC, l), ss = gf(p, G_SS, l), s2 = gf(p, G_S2TH, l), c2 = gf(p, G_C2TH, l);
-    m.mxx = Mxx * cc + Myy * ss - Mxy * s2;
-    m.myy = Mxx * ss + Myy * cc + Mxy * s2;
-    m.mxy = (Mxx - Myy) * 0.5 * s2 + Mxy * c2;
-}
-
 // Unrotated closure with Cramer's rule (2d_mrlbm.f90:1496-1633, 1974-2003) for a generic
 // scalar, as closure_unrotated in step_fp64.cuh.
 template <class P, class S>
@@ -359,58 +309,35 @@ __device__ __forceinline__ void closure_unrotated_s(const P& p, int l, const S f
     m.mxy = Mxy;
 }
 
-// Curved-wall node l from its own inputs f and its 8 stencil nodes' (u, v, mx, my): bilinear
-// interpolation at reference points 2 and 3, extrapolation to the node, the closure the case
-// selects, collision (2d_mrlbm.f90:294-311, 768-928, 1496-2003, 407-457; the order of
-// boundary_close_core in step_fp64.cuh) and the node's drag term (2d_mrlbm.f90:558-591).
-// The eight stencil nodes' u, v and rotated moments come as plain values (qd[kind][t]); the
-// one stencil node s whose inputs carry the derivative (s < 0: none) comes as duals.  Each
-// operand is formed where it is used, so no per-thread array of stencil duals exists.
-template <int CL, class P, class S>
-__device__ __forceinline__ void wall_map(const P& p, int l, const S f[Q], const double (*qd)[8], int s, S us, S vs,
-                                         S mxs, S mys, S fo[Q], S& drag) {
-    auto val = [&](int kind, int t) -> S {
-        if (t == s) return kind == 0 ? us : kind == 1 ? vs : kind == 2 ? mxs : mys;
-        return S(qd[kind][t]);
-    };
-    S u[2], v[2], mx[2], my[2];
+// Curved-wall node l with the unrotated closure, from its own inputs f and its 8 stencil nodes' (u, v):
+// bilinear interpolation at reference points 2 and 3, extrapolation to the node, closure, collision
+// (2d_mrlbm.f90:294-311, 768-819, 1496-1633, 407-457) and the node's drag term (2d_mrlbm.f90:558-591).
+// The eight stencil nodes' u and v come as plain values (qd[kind][t]); the one stencil node s whose
+// inputs carry the derivative (s < 0: none) comes as duals.  Each operand is formed where it is used,
+// so no per-thread array of stencil duals exists.
+template <class P, class S>
+__device__ __forceinline__ void wall_map_unrotated(const P& p, int l, const S f[Q], const double (*qd)[8], int s, S us, S vs,
+                                                   S fo[Q], S& drag) {
+    auto val = [&](int kind, int t) -> S { return t == s ? (kind == 0 ? us : vs) : S(qd[kind][t]); };
+    S u[2], v[2];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         const double xd = gf(p, r == 0 ? G_XD2 : G_XD3, l), yd = gf(p, r == 0 ? G_YD2 : G_YD3, l);
-        S row_u[2], row_v[2], row_mx[2], row_my[2];
+        S row_u[2], row_v[2];
 #pragma unroll
         for (int rr = 0; rr < 2; ++rr) {
             const int s0 = 4 * r + 2 * rr;
             row_u[rr] = (1.0 - xd) * val(0, s0) + xd * val(0, s0 + 1);
             row_v[rr] = (1.0 - xd) * val(1, s0) + xd * val(1, s0 + 1);
-            row_mx[rr] = (1.0 - xd) * val(2, s0) + xd * val(2, s0 + 1);
-            row_my[rr] = (1.0 - xd) * val(3, s0) + xd * val(3, s0 + 1);
         }
         u[r] = (1.0 - yd) * row_u[0] + yd * row_u[1];
         v[r] = (1.0 - yd) * row_v[0] + yd * row_v[1];
-        mx[r] = (1.0 - yd) * row_mx[0] + yd * row_mx[1];
-        my[r] = (1.0 - yd) * row_my[0] + yd * row_my[1];
     }
     const double t2 = gf(p, G_T2, l), t3 = gf(p, G_T3, l);
-    constexpr bool rotated = CL != CLOSURE_UNROTATED;
-    // the node's own moments survive only where no closure or extrapolation replaces them
     MacS<S> m;
-    if (CL == CLOSURE_NONE || (rotated && !p.vel_interp)) m = moments_s(f, p.hm, p.hp);
-    if (!rotated || p.vel_interp) {
-        m.ux = t2 * u[0] - t3 * u[1];
-        m.uy = t2 * v[0] - t3 * v[1];
-    }
-    S Mxx = 0.0, Myy = 0.0;
-    if (rotated && p.mom_interp) {
-        Mxx = t2 * mx[0] - t3 * mx[1];
-        Myy = t2 * my[0] - t3 * my[1];
-    }
-    if constexpr (CL == CLOSURE_UNROTATED) {
-        closure_unrotated_s(p, l, f, m.ux, m.uy, m);
-    } else if constexpr (CL != CLOSURE_NONE) {
-        const double c = gf(p, G_CTH, l), sn = gf(p, G_STH, l);
-        closure_rotated_s<CL>(p, l, f, m.ux * c + m.uy * sn, m.uy * c - m.ux * sn, Mxx, Myy, m);
-    }
+    m.ux = t2 * u[0] - t3 * u[1];
+    m.uy = t2 * v[0] - t3 * v[1];
+    closure_unrotated_s(p, l, f, m.ux, m.uy, m);
     collide_s(p, m, fo);
     const int Is = gi(p, I_IS, l), Os = gi(p, I_OS, l);
     S fxo = 0.0, fxi = 0.0;
@@ -555,8 +482,8 @@ __device__ __forceinline__ void adjoint_edge(const P& p, const AdjArgs& a, int e
     if (q > 9 && !outlet) return;
     if (q == 9 && !outlet && !inlet) return;
     double g[Q], gn[Q];
-    gather_d(p, i, j, g);
-    if (outlet) gather_d(p, nx - 1, j, gn);
+    edge_gather_d(p, i, j, g);
+    if (outlet) edge_gather_d(p, nx - 1, j, gn);
     Dual f[Q], fn[Q];
 #pragma unroll
     for (int k = 0; k < Q; ++k) {
@@ -576,12 +503,12 @@ __device__ __forceinline__ void adjoint_edge(const P& p, const AdjArgs& a, int e
     if (q == 0 && p.body) body_grad(p, a, i, j, lam);
 }
 
-// Curved-wall node l, one block: the block stages the node's 81 inputs (9 own, 9 for each of
-// its 8 stencil nodes) and the stencil quantities in shared memory; thread q < 81 then runs
+// Curved-wall node l with the unrotated closure, one block: the block stages the node's 81 inputs (9 own, 9 for each
+// of its 8 stencil nodes) and the stencil quantities in shared memory; thread q < 81 then runs
 // the node's map with the derivative along input q (only its stencil node's quantities carry
 // a derivative) and scatters the contracted column.
-template <int CL, class P>
-__device__ __forceinline__ void adjoint_wall(const P& p, const AdjArgs& a, int l) {
+template <class P>
+__device__ __forceinline__ void adjoint_wall_unrotated(const P& p, const AdjArgs& a, int l) {
     __shared__ double in[81], lam[Q], qd[4][8];
     __shared__ int slot[81];
     const int q = threadIdx.x;
@@ -628,11 +555,206 @@ __device__ __forceinline__ void adjoint_wall(const P& p, const AdjArgs& a, int l
         stencil_quad(p, l, s, g, us, vs, mxs, mys);    // only stencil s depends on input q
     }
     Dual fo[Q], drag;
-    wall_map<CL>(p, l, f, qd, s, us, vs, mxs, mys, fo, drag);
+    wall_map_unrotated(p, l, f, qd, s, us, vs, fo, drag);
     double c = a.wJ * drag.d;
 #pragma unroll
     for (int k = 0; k < Q; ++k) c += lam[k] * fo[k].d;
     if (slot[q] >= 0) atomicAdd(a.lam_out + slot[q], c);
+}
+
+// Sum over the 16 lanes of a node, in every lane.
+__device__ __forceinline__ double sum16(double v) {
+#pragma unroll
+    for (int d = 8; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d, 16);
+    return v;
+}
+
+// Curved-wall nodes with a rotated closure (strong, weak, rho_eq) or none: reverse mode by hand, 16
+// lanes per node as in the forward step's wall blocks (fp64::wall_block, whose quantities it names
+// alike).  Lane s (and s + 8) holds stencil node s, lane k < 9 direction k; b after a name is the
+// derivative of J by it.  Forward: extrapolated (ux, uy, X, Y) = sum_s kappa_s (stencil quantities),
+// closure (rho, Z), moments rotated back, collision, fo_k, drag.  Then the same backwards; the sums
+// over the directions are shuffles.  Every table value is loaded before the wait.  With dual numbers a
+// block ran the map once for each of the node's 81 inputs: 12 of an adjoint step's 20 us on
+// 512 x 128 (the gradient over 400 steps 11.2 ms, with this form 9.4; the sums in another order,
+// 5e-15 of the largest entry apart).
+template <int CL, class P>
+__device__ __forceinline__ void adjoint_wall(const P& p, const AdjArgs& a, int block) {
+    const int tid = threadIdx.x, lane = tid & 15, nb = p.nb;
+    const int l = block * (int)(blockDim.x >> 4) + (tid >> 4);
+    const bool active = l < nb;
+    const int lt = active ? l : 0;
+    auto G = [&](int field) { return gf(p, field, lt); };
+    const int k = min(lane, Q - 1), s = lane & 7, r = s >> 2;
+    const bool dir = active && lane < Q;
+    const int i = gi(p, I_NODEI, lt), j = gi(p, I_NODEJ, lt), si = gi(p, I_SI + s, lt), sj = gi(p, I_SJ + s, lt);
+    const double in = (gi(p, I_IS, lt) >> k) & 1, out = (gi(p, I_OS, lt) >> k) & 1;
+    const double scc = G(G_SCC + s), sss = G(G_SSS + s), ss2 = G(G_SS2 + s);
+    const double xd = G(r == 0 ? G_XD2 : G_XD3), yd = G(r == 0 ? G_YD2 : G_YD3);
+    const double kappa = (r == 0 ? G(G_T2) : -G(G_T3)) * ((s & 1) ? xd : 1.0 - xd) * ((s & 2) ? yd : 1.0 - yd);
+    const double c = G(G_CTH), sn = G(G_STH), s2 = G(G_S2TH), c2 = G(G_C2TH), cc = G(G_CC), ss = G(G_SS);
+    const double cxp = G(G_CXP + k), cyp = G(G_CYP + k), hxx = G(G_HXXP + k), hyy = G(G_HYYP + k), hxy = G(G_HXYP + k);
+    const double B11 = G(G_B11), B22 = G(G_B22), B12 = G(G_B12), F11 = G(G_F11), F22 = G(G_F22), F12 = G(G_F12);
+    const double exk = ex(k), eyk = ey(k), Hx = exk != 0.0 ? (double)p.hp : (double)p.hm, Hy = eyk != 0.0 ? (double)p.hp : (double)p.hm;
+    const double w = lane < Q ? (double)(k == 0 ? p.w[0] : k < 5 ? p.w[1] : p.w[5]) : 0.0;     // lanes past the directions add nothing
+    const double om = p.omega, om1 = p.omega1;
+    wait_prior_grid();
+
+    const int64_t own = p.L.at(i, j, k), src = p.L.at(i - ex(k), j - ey(k), k);     // wall nodes are interior nodes
+    double f = 0.0, lam = 0.0;
+    fp64::Mac q{};
+    double qs[Q];
+#pragma unroll
+    for (int t = 0; t < Q; ++t) qs[t] = (double)p.w[t];
+    if (active) {
+        typename P::Real g[Q];
+        gather_interior(p, si, sj, g);
+        if (lane < Q) {
+            f = to_f(p, k, __ldg(p.src + src));
+            lam = a.lam_in[own];
+        }
+#pragma unroll
+        for (int t = 0; t < Q; ++t) qs[t] = to_f(p, t, g[t]);
+    }
+    if (dir) a.lam_in[own] = 0.0;
+    q = fp64::moments(qs, p.hm, p.hp);                                               // stencil node s
+    const double xs = q.mxx * scc + q.myy * sss + q.mxy * ss2, ys = q.mxx * sss + q.myy * scc - q.mxy * ss2;
+    const double half = lane < 8 ? 1.0 : 0.0;                                          // each stencil node once
+    double ux = sum16(half * kappa * q.ux), uy = sum16(half * kappa * q.uy);
+    double X = sum16(half * kappa * xs), Y = sum16(half * kappa * ys);
+    if (!p.mom_interp) X = Y = 0.0;
+    // the node's own moments, where something of them survives
+    constexpr bool none = CL == CLOSURE_NONE;
+    MacS<double> m0{1.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    double inv0 = 1.0;
+    if (none || !p.vel_interp) {
+        m0.rho = sum16(f);
+        inv0 = 1.0 / m0.rho;
+        m0.ux = sum16(f * exk) * inv0;
+        m0.uy = sum16(f * eyk) * inv0;
+        m0.mxx = sum16(f * Hx) * inv0;
+        m0.myy = sum16(f * Hy) * inv0;
+        m0.mxy = sum16(f * exk * eyk) * inv0;
+    }
+    if (!p.vel_interp) { ux = m0.ux; uy = m0.uy; }
+    const double up = ux * c + uy * sn, vp = uy * c - ux * sn;
+    double rho, mxx, myy, mxy;
+    double A_p = 0.0, E_p = 0.0, rhoI = 1.0, mI = 0.0, D = 0.0, Z = 0.0, Pp = 0.0, den = 1.0, L11 = 0.0, L22 = 0.0, L12 = 1.0;
+    constexpr bool strong = CL == CLOSURE_STRONG, weak = CL == CLOSURE_WEAK;
+    const double beta = strong ? om1 : 1.0;
+    if constexpr (none) {
+        rho = m0.rho; mxx = m0.mxx; myy = m0.myy; mxy = m0.mxy;
+    } else {
+        const double A = w * (1.0 + 3.0 * up * cxp + 3.0 * vp * cyp);
+        const double E = A + w * (4.5 * up * up * hxx + 4.5 * vp * vp * hyy + 9.0 * up * vp * hxy);
+        rhoI = sum16(in * f);
+        mI = sum16(in * f * hxy) / rhoI;
+        D = sum16(in * A * hxy);
+        if (strong || weak) A_p = sum16((strong ? out : in) * A);
+        if (!weak) E_p = sum16((strong ? out : in) * E);
+        if constexpr (strong || weak) {
+            Pp = strong ? om1 * A_p + om * E_p : A_p;
+            L11 = beta * B11 * mI - F11;
+            L22 = beta * B22 * mI - F22;
+            L12 = 2.0 * (beta * B12 * mI - F12);
+            Z = (D - Pp * mI - X * L11 - Y * L22) / L12;
+            den = Pp + beta * (X * B11 + Y * B22 + 2.0 * Z * B12);
+        } else {
+            L11 = F11; L22 = F22; L12 = 2.0 * F12;
+            Z = (E_p * mI - D - X * L11 - Y * L22) / L12;
+            den = E_p;
+        }
+        rho = rhoI / den;
+        mxx = X * cc + Y * ss - Z * s2;
+        myy = X * ss + Y * cc + Z * s2;
+        mxy = (X - Y) * 0.5 * s2 + Z * c2;
+    }
+    // collision and reconstruction of direction k
+    double xx = om1 * mxx + om * ux * ux, yy = om1 * myy + om * uy * uy;
+    const double xy = om1 * mxy + om * ux * uy;
+    if (p.incomp_bulk) {
+        const double t = 0.5 * (((xx + yy) - ux * ux) - uy * uy);
+        xx -= t;
+        yy -= t;
+    }
+    const double Phi = 1.0 + 3.0 * (exk * ux + eyk * uy) + 4.5 * xx * Hx + 4.5 * yy * Hy + 9.0 * xy * exk * eyk;
+
+    // ---- backwards: fo_k = w rho Phi, drag = sum_in f e_x - sum_out fo e_x
+    const double lw = (lam - a.wJ * out * exk) * w, lr = lw * rho;
+    double rb = sum16(lw * Phi), uxb = sum16(3.0 * exk * lr), uyb = sum16(3.0 * eyk * lr);
+    double xxb = sum16(4.5 * Hx * lr), yyb = sum16(4.5 * Hy * lr);
+    const double xyb = sum16(9.0 * exk * eyk * lr);
+    if (p.incomp_bulk) {
+        const double tb = -(xxb + yyb);
+        xxb += 0.5 * tb;
+        yyb += 0.5 * tb;
+        uxb -= tb * ux;
+        uyb -= tb * uy;
+    }
+    uxb += om * (2.0 * ux * xxb + uy * xyb);
+    uyb += om * (2.0 * uy * yyb + ux * xyb);
+    const double mxxb = om1 * xxb, myyb = om1 * yyb, mxyb = om1 * xyb;
+    double fb = a.wJ * in * exk, Xb = 0.0, Yb = 0.0;
+    if constexpr (!none) {
+        Xb = mxxb * cc + myyb * ss + 0.5 * mxyb * s2;
+        Yb = mxxb * ss + myyb * cc - 0.5 * mxyb * s2;
+        double Zb = (myyb - mxxb) * s2 + mxyb * c2;
+        double rhoIb = rb / den;
+        const double denb = -rb * rho / den;
+        double mIb, Db, Ab, Eb;                        // Ab, Eb: by this direction's A and E
+        if constexpr (strong || weak) {
+            Xb += denb * beta * B11;
+            Yb += denb * beta * B22;
+            Zb += 2.0 * denb * beta * B12;
+            const double t = Zb / L12;
+            Xb -= t * L11;
+            Yb -= t * L22;
+            mIb = -beta * t * (X * B11 + Y * B22 + 2.0 * Z * B12) - t * Pp;
+            const double Pb = denb - t * mI;
+            Db = t;
+            Ab = in * Db * hxy + (strong ? out * om1 * Pb : in * Pb);
+            Eb = strong ? out * om * Pb : 0.0;
+        } else {
+            const double t = Zb / L12;
+            Xb -= t * L11;
+            Yb -= t * L22;
+            mIb = t * E_p;
+            Db = -t;
+            Ab = in * Db * hxy;
+            Eb = in * (denb + t * mI);
+        }
+        rhoIb -= mIb * mI / rhoI;
+        fb += in * (rhoIb + mIb / rhoI * hxy);
+        const double both = 3.0 * w * (Ab + Eb), e9 = 9.0 * w * Eb;
+        const double upb = sum16(both * cxp + e9 * (up * hxx + vp * hxy)), vpb = sum16(both * cyp + e9 * (vp * hyy + up * hxy));
+        uxb += upb * c - vpb * sn;
+        uyb += upb * sn + vpb * c;
+    }
+    if (none || !p.vel_interp) {                       // through the node's own moments
+        double t = 0.0;
+        if (none) t += rb + inv0 * (mxxb * (Hx - m0.mxx) + myyb * (Hy - m0.myy) + mxyb * (exk * eyk - m0.mxy));
+        if (!p.vel_interp) t += inv0 * (uxb * (exk - m0.ux) + uyb * (eyk - m0.uy));
+        fb += t;
+    }
+    if (dir) atomicAdd(a.lam_out + src, fb);
+    // through the stencil nodes
+    const double kv = p.vel_interp ? kappa : 0.0, km = !none && p.mom_interp ? kappa : 0.0;
+    if (active && lane < 8 && (kv != 0.0 || km != 0.0)) {
+        const double inv = 1.0 / q.rho, ub = kv * uxb * inv, vb = kv * uyb * inv;
+        const double ax = km * (Xb * scc + Yb * sss) * inv, ay = km * (Xb * sss + Yb * scc) * inv, axy = km * (Xb - Yb) * ss2 * inv;
+        double* d = a.lam_out + p.L.at(si, sj, 0);
+#pragma unroll
+        for (int t = 0; t < Q; ++t) {
+            const double hx = ex(t) != 0 ? (double)p.hp : (double)p.hm, hy = ey(t) != 0 ? (double)p.hp : (double)p.hm;
+            atomicAdd(d + t * p.L.plane - ey(t) * (int64_t)p.L.pitch - ex(t),
+                      ub * (ex(t) - q.ux) + vb * (ey(t) - q.uy) + ax * (hx - q.mxx) + ay * (hy - q.myy) + axy * (ex(t) * ey(t) - q.mxy));
+        }
+    }
+}
+
+// Wall blocks of 128 threads: a node each with the unrotated closure, eight nodes otherwise.
+__host__ __device__ inline int adjoint_wall_blocks(int closure, int nb) {
+    return closure == CLOSURE_UNROTATED ? nb : (nb + 7) / 8;
 }
 
 // One adjoint step as two launches, ordered like the forward step's (step_common.cuh): the
@@ -642,15 +764,20 @@ __device__ __forceinline__ void adjoint_wall(const P& p, const AdjArgs& a, int l
 // waits for the first launch, so the step completes as a whole.
 template <class P, int CL>
 __global__ void __launch_bounds__(128) adjoint_aux(const __grid_constant__ P p, const __grid_constant__ AdjArgs a) {
-    wait_prior_grid();
-    const int b = (int)blockIdx.x;
-    if (b < p.nb) {
-        adjoint_wall<CL>(p, a, b);
+    const int b = (int)blockIdx.x, nw = adjoint_wall_blocks(CL, p.nb);
+    if (b < nw) {
+        if constexpr (CL == CLOSURE_UNROTATED) {
+            wait_prior_grid();
+            adjoint_wall_unrotated(p, a, b);
+        } else {
+            adjoint_wall<CL>(p, a, b);
+        }
         return;
     }
+    wait_prior_grid();
     // lambda^n of the block's 7 edge nodes, staged once and cleared for reuse
     __shared__ double lam[7][Q];
-    const int t = threadIdx.x, e0 = 7 * (b - p.nb);
+    const int t = threadIdx.x, e0 = 7 * (b - nw);
     if (t < 7 * Q) {
         const int e = e0 + t / Q, k = t % Q;
         if (e < a.n_edge) {

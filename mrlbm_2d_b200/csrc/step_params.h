@@ -40,6 +40,7 @@ struct OvrEntry { int i, j, k, pad; double v; };
 
 template <class T>
 struct alignas(64) StepParams {
+    using Real = T;
     CUtensorMap tmap;             // 2-D map of src (rows = 9 planes x (ny+2)), TMA shapes only
     CUtensorMap tmap_st;          // 2-D map of dst with the store box (BX x BY), TMA-store shapes only
     unsigned long long* tile_ctr; // tile claim counter of the TMA shapes
