@@ -771,7 +771,16 @@ int replay_graph(mrlbm_handle* h, int n, bool fields, mrlbm_handle::Replay*& out
     return MRLBM_OK;
 }
 
+// This thread's calls as they would be were no other thread capturing: a graph being captured elsewhere in
+// the process (torch captures in the global mode) otherwise forbids the allocations and copies below.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 int step_replay(mrlbm_handle* h, int n) {
+    RelaxedCapture relaxed;
     const int z = h->iter + n;
     const bool fields = fields_at(h, h->iter + 1);
     mrlbm_handle::Replay* g = nullptr;
