@@ -67,9 +67,11 @@ __device__ __forceinline__ Dual operator+(Dual a, Dual b) { return Dual(a.v + b.
 __device__ __forceinline__ Dual operator-(Dual a, Dual b) { return Dual(a.v - b.v, a.d - b.d); }
 __device__ __forceinline__ Dual operator-(Dual a) { return Dual(-a.v, -a.d); }
 __device__ __forceinline__ Dual operator*(Dual a, Dual b) { return Dual(a.v * b.v, a.d * b.v + a.v * b.d); }
+// (one division each, a reciprocal: a division is some 40 instructions, and the edge nodes' maps divide
+// seven times in a row)
 __device__ __forceinline__ Dual operator/(Dual a, Dual b) {
-    const double q = a.v / b.v;
-    return Dual(q, (a.d - q * b.d) / b.v);
+    const double r = 1.0 / b.v, q = a.v * r;
+    return Dual(q, (a.d - q * b.d) * r);
 }
 __device__ __forceinline__ Dual operator+(Dual a, double b) { return Dual(a.v + b, a.d); }
 __device__ __forceinline__ Dual operator+(double a, Dual b) { return Dual(a + b.v, b.d); }
@@ -77,10 +79,13 @@ __device__ __forceinline__ Dual operator-(Dual a, double b) { return Dual(a.v - 
 __device__ __forceinline__ Dual operator-(double a, Dual b) { return Dual(a - b.v, -b.d); }
 __device__ __forceinline__ Dual operator*(Dual a, double b) { return Dual(a.v * b, a.d * b); }
 __device__ __forceinline__ Dual operator*(double a, Dual b) { return Dual(a * b.v, a * b.d); }
-__device__ __forceinline__ Dual operator/(Dual a, double b) { return Dual(a.v / b, a.d / b); }
+__device__ __forceinline__ Dual operator/(Dual a, double b) {
+    const double r = 1.0 / b;
+    return Dual(a.v * r, a.d * r);
+}
 __device__ __forceinline__ Dual operator/(double a, Dual b) {
-    const double q = a / b.v;
-    return Dual(q, -q * b.d / b.v);
+    const double r = 1.0 / b.v, q = a * r;
+    return Dual(q, -q * b.d * r);
 }
 
 template <class S>
@@ -400,8 +405,14 @@ __device__ __forceinline__ void adjoint_bulk(const P& p, const AdjArgs& a, int t
         gbx = a.grad_body[n];
         gby = a.grad_body[N + n];
     }
+    // the buffer becomes step n-2's target: cleared where some of the nine nodes that pull these slots add to it,
+    // left where all of them store (a fifth of the node's traffic)
+    const bool keep = i > 2 && i < nx - 2 && j > 2 && j < ny - 1 &&
+                      (i < a.sx0 - 1 || i > a.sx1 + 1 || j < a.sy0 - 1 || j > a.sy1 + 1);
+    if (!keep) {
 #pragma unroll
-    for (int k = 0; k < Q; ++k) a.lam_in[own + k * plane] = 0.0;   // read once: the buffer becomes step n-2's target
+        for (int k = 0; k < Q; ++k) a.lam_in[own + k * plane] = 0.0;
+    }
     const fp64::Mac m = fp64::moments(g, p.hm, p.hp);
     const bool u_zero = cls == CLS_SOLID && p.zero_solid_u;
     const double ux = u_zero ? 0.0 : m.ux, uy = u_zero ? 0.0 : m.uy;
@@ -470,27 +481,49 @@ __device__ __forceinline__ void adjoint_bulk(const P& p, const AdjArgs& a, int t
     }
 }
 
-// Edge nodes: thread (e, q), e over the n_edge nodes of edge_node_ij, q over 18 inputs: own
-// inputs 0..8; at the outlet the copied neighbour's inputs 9..17; at the inlet q = 9 is u_in(j).
+// Edge block b: 7 nodes of edge_node_ij x 18 threads, thread q of a node for its input q: own inputs
+// 0..8; at the outlet the copied neighbour's inputs 9..17; at the inlet q = 9 is u_in(j).  Every load
+// (the nodes' lambda^n, staged once and cleared for reuse, and each thread's inputs) is issued before
+// the first use: with the staging ahead of the gathers and two divisions per dual division these blocks
+// were the last of a step to end, 7.4 of its 8.4 us on 512 x 128 (the gradient over 400 steps 9.1 ms;
+// with this, and without the clearing of what adjoint_bulk stores outright, 8.1).
 template <class P>
-__device__ __forceinline__ void adjoint_edge(const P& p, const AdjArgs& a, int e, int q, const double* lam) {
-    if (e >= a.n_edge) return;
-    const int nx = p.L.nx;
-    int i, j;
-    edge_node_ij(p, e, i, j);
+__device__ __forceinline__ void adjoint_edge_block(const P& p, const AdjArgs& a, int b) {
+    __shared__ double lams[7][Q];
+    const int t = threadIdx.x, nx = p.L.nx;
+    double* clear = nullptr;
+    double lv = 0.0;
+    if (t < 7 * Q && 7 * b + t / Q < a.n_edge) {
+        int i, j;
+        edge_node_ij(p, 7 * b + t / Q, i, j);
+        clear = a.lam_in + p.L.at(i, j, t % Q);
+        lv = *clear;
+    }
+    const int e = 7 * b + t / 18, q = t % 18;
+    int i = 0, j = 0;
+    bool on = t < 7 * 18 && e < a.n_edge;
+    if (on) edge_node_ij(p, e, i, j);
     const bool inlet = i == 1, outlet = i == nx;
-    if (q > 9 && !outlet) return;
-    if (q == 9 && !outlet && !inlet) return;
-    double g[Q], gn[Q];
-    edge_gather_d(p, i, j, g);
-    if (outlet) edge_gather_d(p, nx - 1, j, gn);
+    on = on && (outlet || q < 9 || (inlet && q == 9));
+    double g[Q] = {}, gn[Q] = {}, u0 = 0.0;
+    if (on) {
+        edge_gather_d(p, i, j, g);
+        if (outlet) edge_gather_d(p, nx - 1, j, gn);
+        u0 = p.u_in ? (double)p.u_in[j - 1] : (double)p.uinlet;
+    }
+    if (clear) {
+        lams[t / Q][t % Q] = lv;
+        *clear = 0.0;
+    }
+    __syncthreads();
+    if (!on) return;
+    const double* lam = lams[t / 18];
     Dual f[Q], fn[Q];
 #pragma unroll
     for (int k = 0; k < Q; ++k) {
         f[k] = Dual(g[k], q == k ? 1.0 : 0.0);
-        fn[k] = Dual(outlet ? gn[k] : 0.0, (outlet && q == 9 + k) ? 1.0 : 0.0);
+        fn[k] = Dual(gn[k], (outlet && q == 9 + k) ? 1.0 : 0.0);
     }
-    const double u0 = p.u_in ? (double)p.u_in[j - 1] : (double)p.uinlet;
     const Dual uin(u0, (inlet && q == 9) ? 1.0 : 0.0);
     Dual fo[Q];
     edge_map(p, i, j, f, fn, uin, fo);
@@ -763,7 +796,7 @@ __host__ __device__ inline int adjoint_wall_blocks(int closure, int nb) {
 // first launch has waited for the previous step and run beside it; the last bulk block to finish
 // waits for the first launch, so the step completes as a whole.
 template <class P, int CL>
-__global__ void __launch_bounds__(128) adjoint_aux(const __grid_constant__ P p, const __grid_constant__ AdjArgs a) {
+__global__ void __launch_bounds__(128, 3) adjoint_aux(const __grid_constant__ P p, const __grid_constant__ AdjArgs a) {
     const int b = (int)blockIdx.x, nw = adjoint_wall_blocks(CL, p.nb);
     if (b < nw) {
         if constexpr (CL == CLOSURE_UNROTATED) {
@@ -775,21 +808,7 @@ __global__ void __launch_bounds__(128) adjoint_aux(const __grid_constant__ P p, 
         return;
     }
     wait_prior_grid();
-    // lambda^n of the block's 7 edge nodes, staged once and cleared for reuse
-    __shared__ double lam[7][Q];
-    const int t = threadIdx.x, e0 = 7 * (b - nw);
-    if (t < 7 * Q) {
-        const int e = e0 + t / Q, k = t % Q;
-        if (e < a.n_edge) {
-            int i, j;
-            edge_node_ij(p, e, i, j);
-            const int64_t at = p.L.at(i, j, k);
-            lam[t / Q][k] = a.lam_in[at];
-            a.lam_in[at] = 0.0;
-        }
-    }
-    __syncthreads();
-    if (t < 126) adjoint_edge(p, a, e0 + t / 18, t % 18, lam[t / 18]);
+    adjoint_edge_block(p, a, b - nw);
 }
 
 template <class P>

@@ -1921,10 +1921,11 @@ extern "C" int mrlbm_adjoint_drag(mrlbm_handle* h, int32_t nsteps, int32_t windo
     // sweep segment c + 1 from the other set on the handle's stream: a recompute waits for the
     // sweep that last used its set, a sweep for the recompute of its segment.
     std::vector<void*>* sets[2] = {&seg, &seg2};
-    int sx0 = h->L.nx + 1, sx1 = 0, sy0 = h->L.ny + 1, sy1 = 0;   // stencil-node bounding box
+    int sx0 = h->L.nx + 1, sx1 = 0, sy0 = h->L.ny + 1, sy1 = 0;   // bounding box of the wall nodes (m = 12) and their stencil nodes
     for (int l = 0; l < h->geo.nb; ++l)
-        for (int m = 0; m < 12; ++m) {
-            const int si = h->geo.tint[(size_t)(I_SI + m) * h->geo.nb + l], sj = h->geo.tint[(size_t)(I_SJ + m) * h->geo.nb + l];
+        for (int m = 0; m <= 12; ++m) {
+            const int si = h->geo.tint[(size_t)(m < 12 ? I_SI + m : I_NODEI) * h->geo.nb + l];
+            const int sj = h->geo.tint[(size_t)(m < 12 ? I_SJ + m : I_NODEJ) * h->geo.nb + l];
             sx0 = std::min(sx0, si); sx1 = std::max(sx1, si); sy0 = std::min(sy0, sj); sy1 = std::max(sy1, sj);
         }
     cudaStream_t rs = nullptr;
