@@ -105,7 +105,7 @@ struct mrlbm_handle {
         uint64_t used = 0;
     } replay[N_REPLAYS];
     uint64_t replay_clock = 0;
-    int64_t stepped = 0;                      // steps taken by the handle
+    int64_t stepped = 0;                      // steps taken by the handle, the autotuner's left out
     bool no_replay = false;                   // autotuner trials of single shapes
     int* d_call = nullptr;                    // call state of the replay (StepParams::call)
     std::vector<OvrEntry> ovr;                // loaded-state overrides (see OvrEntry)
@@ -483,6 +483,7 @@ int launch_one(mrlbm_handle* h, bool stats, bool plot, bool macro) {
     h->launches += nl;
     if (rc == -2) {
         h->launches -= nl;
+        h->tmap_cfg = -1;
         return fail(h, MRLBM_EUNSUPPORTED, "tile shape does not fit this precision");
     }
     if (rc != 0) {
@@ -516,10 +517,11 @@ bool pairs_possible(const mrlbm_handle* h) {
     return !h->halo_l && !h->halo_r && h->L.nx >= PAIR_MIN_NX && h->L.ny >= PAIR_MIN_NY;
 }
 
-// Whether pairs are taken from the start (the autotuner measures instead).  Below about a million FP64 or
-// two million FP32 nodes a step is bound by the wall nodes' latency and the launches, of which a pair
-// has as many.  Single steps and pairs, us per step: 1003 x 251 8.5 and 10.5 (FP64), 8.0 and 11.4 (FP32);
-// 2048 x 512 25.9 and 20.3, 11.4 and 13.2; 2900 x 725 50.8 and 35.4, 27.3 and 21.0; 4099 x 1023 97 and 63, 52 and 37.
+// Whether pairs are taken from the start (the autotuner measures instead).  On smaller lattices a step is
+// bound by its chain of wall nodes and launches, which a pair does not shorten, and the wider skirt of a
+// two-step tile weighs more.  Single steps and pairs, us per step, FP64 and FP32: 1003 x 251 5.7 and 6.8, 5.5 and 5.7;
+// 1400 x 350 9.0 and 10.9, 6.4 and 7.2; 2048 x 512 25.4 and 19.7, 11.2 and 11.8; 2900 x 725 50.8 and 33.9, 27.3 and
+// 20.9; 4099 x 1023 97 and 61.5, 52 and 36.7.
 bool pairs_pay(const mrlbm_handle* h) {
     const int64_t nodes = (int64_t)h->L.nx * h->L.ny;
     return std::min(h->L.nx, h->L.ny) >= 64 && nodes >= (h->precision == MRLBM_FP64 ? 700000 : 1500000);
@@ -591,10 +593,11 @@ bool fields_at(const mrlbm_handle* h, int iter) { return h->d_fstat && iter >= h
 
 // Whether the next two steps can be one pair: no loaded-state overrides, no surface record, both
 // steps or neither inside the field-statistics window, room for both records in the ring.
+// A TMA shape newly set is taken by a single step first, which refuses those that do not fit the precision.
 bool pair_ok(const mrlbm_handle* h) {
     const int a = h->iter + 1, b = h->iter + 2;
-    return h->pairs && !h->ovr_live && h->ring_n + 2 <= RING_CAP && fields_at(h, a) == fields_at(h, b) &&
-           !(h->surf_on && (stats_at(h, a) || stats_at(h, b)));
+    return h->pairs && (!is_tma_cfg(h->tile_cfg) || h->tmap_cfg == h->tile_cfg) && !h->ovr_live &&
+           h->ring_n + 2 <= RING_CAP && fields_at(h, a) == fields_at(h, b) && !(h->surf_on && (stats_at(h, a) || stats_at(h, b)));
 }
 
 // Parameters of a step of the handle but for its time levels and record.
@@ -662,6 +665,7 @@ int launch_two(mrlbm_handle* h) {
 // and replayed: 80 x 50 FP64 2100, 1620; 400 x 100 2100, 1690 (FP32 1520, 1395); 1003 x 251 2690, 2420
 // (FP32 2295, 2210); 1400 x 350 the same, its steps outlast their launches.
 constexpr int64_t REPLAY_MAX_NODES = 400000;
+constexpr int REPLAY_AFTER = 24;
 
 // Length of the run to replay for the next `left` steps, or 0: launched steps.  Every step of the run must be
 // one whose launch differs from its captured form in the call state only.
@@ -673,9 +677,9 @@ int replay_length(const mrlbm_handle* h, int left) {
     for (int n : REPLAY_STEPS) {
         const int a = h->iter + 1, z = h->iter + n;
         if (left < n || h->ring_n + n > RING_CAP) continue;
-        // a graph costs its first call about as much as 2 n launched steps would take: not for calls or
-        // handles that end before it has paid (0.3 ms for 16 and 0.6 ms for 64 steps, measured)
-        if (left < 3 * n && h->stepped < 8 * n) continue;
+        // capturing costs 0.3 ms for 16 and 0.7 ms for 64 steps, a replayed step saves 0.5 to 1.2 us: not
+        // before the handle has been asked for the steps that pay for it
+        if (h->stepped + left < REPLAY_AFTER * n) continue;
         const bool fields = h->d_fstat && std::max(a, h->fstat_begin) <= std::min(z, h->fstat_end);
         if (fields && !(h->fstat_begin <= a && z <= h->fstat_end)) continue;       // all of the run or none of it
         // a plot step's solid velocities follow the call state in the tile shapes only
@@ -1701,10 +1705,13 @@ int mrlbm_autotune(mrlbm_handle* h, int32_t trial_steps, int32_t* best_cfg, doub
     int best = cfg0;
     float best_t = 1e30f;
     int rc = MRLBM_OK;
-    // every shape by single steps, then (index N_ALL_CFGS) the best of them with its steps in pairs
+    // every shape by single steps, then (index N_ALL_CFGS) the best of them with its steps in pairs, on
+    // lattices that are not so small that single steps were always the faster (pairs_pay)
     const bool pairs0 = h->pairs;
+    const int64_t stepped0 = h->stepped;
     h->no_replay = true;
-    const int last = h->pairs_fixed || std::min(h->L.nx, h->L.ny) < 64 ? N_ALL_CFGS : N_ALL_CFGS + 1;
+    const bool try_pairs = !h->pairs_fixed && std::min(h->L.nx, h->L.ny) >= 64 && (int64_t)h->L.nx * h->L.ny > REPLAY_MAX_NODES;
+    const int last = try_pairs ? N_ALL_CFGS + 1 : N_ALL_CFGS;
     bool pairs_best = false;
     for (int c = 0; c < last && rc == MRLBM_OK; ++c) {
         const bool paired = c == N_ALL_CFGS;
@@ -1758,6 +1765,7 @@ int mrlbm_autotune(mrlbm_handle* h, int32_t trial_steps, int32_t* best_cfg, doub
     cudaStreamSynchronize(h->stream);
     cleanup();
     h->no_replay = false;
+    h->stepped = stepped0;
     if (rc != MRLBM_OK) {
         h->tile_cfg = cfg0;
         h->pairs = pairs0;

@@ -148,3 +148,23 @@ def test_batch_streams_in_pairs(mrlbm, monkeypatch, prec):
         assert np.array_equal(c.macro()["ux"], s.macro()["ux"])
         s.close()
     b.close()
+
+
+@pytest.mark.parametrize("prec", [64, 32])
+def test_pairs_refuse_the_shapes_single_steps_refuse(mrlbm, monkeypatch, prec):
+    cfg = cylinder_case(124, 45, 10, 41, 22.5, 80.0, 0.05, seed=2, noise=1e-2)
+    seen = []
+    for pairs in ("0", "1"):
+        monkeypatch.setenv("MRLBM_PAIRS", pairs)
+        s = mrlbm.Simulation(cfg, precision=prec)
+        refused = []
+        for tile in range(mrlbm.N_TILE_CONFIGS):
+            s.tile_config = tile
+            for n in (2, 5):
+                try:
+                    s.step(n)
+                except mrlbm.MrlbmError:
+                    refused.append((tile, n))
+        seen.append((refused, s.iter, s.get_state()))
+        s.close()
+    assert seen[0][:2] == seen[1][:2] and np.array_equal(seen[0][2], seen[1][2])

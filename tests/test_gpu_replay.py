@@ -1,4 +1,4 @@
-"""Runs of steps replayed from captured graphs (calls of 48 steps and more) give the bits of steps launched
+"""Runs of steps replayed from captured graphs (from 384 steps of a handle on 16, from 1536 on 64 at a time) give the bits of steps launched
 one call at a time: populations, every force record and field statistics, whatever begins or ends inside a run."""
 import numpy as np
 import pytest
@@ -41,10 +41,10 @@ def test_replayed_runs_equal_launched_steps(mrlbm, monkeypatch, prec, pairs, nam
     monkeypatch.setenv("MRLBM_PAIRS", pairs)
     cfg = CASES[name]()
     if cfg.post_process:
-        cfg = cfg.replace(statsbegin=50, statsend=215)         # records begin and end inside runs
+        cfg = cfg.replace(statsbegin=50, statsend=2615)        # records begin and end inside runs
 
     def script(s, go):
-        go(200)                                                # 64, then 16 a run, then single steps
+        go(2600)                                               # 64, then 16 a run, then single steps
         out = _out(s)
         go(47)                                                 # an odd count: the other time level
         go(64)
@@ -63,11 +63,13 @@ def test_replayed_runs_with_changing_inputs(mrlbm, monkeypatch, prec, pairs):
     profile = cfg.uo * (1.0 + 0.1 * rng.standard_normal(cfg.ny))
 
     def script(s, go):
-        s.field_stats_window(70, 150)                          # opens and closes inside runs
+        go(700)
+        out = _out(s)
+        s.field_stats_window(740, 840)                         # opens and closes inside runs
         go(160)
-        out = _out(s, fields=True)
+        out += _out(s, fields=True)
         s.set_body_force(body)
-        s.field_stats_window(161, 10000)
+        s.field_stats_window(861, 10000)
         go(130)
         s.set_inlet_profile(profile)
         go(130)
@@ -93,7 +95,7 @@ def test_replayed_runs_of_every_kind_of_tile(mrlbm, prec, tile):
 
     def script(s, go):
         s.tile_config = tile
-        go(150)
+        go(700)
         return _out(s)
 
     _both(mrlbm, cfg, prec, script)
@@ -112,7 +114,7 @@ def test_steps_inside_a_callers_capture_are_launched(mrlbm):
         st = torch.cuda.Stream()
         s = mrlbm.Simulation(cfg, precision=64)
         s.set_stream(st.cuda_stream)
-        s.step(256)
+        s.step(2560)
         s.forces()
         if captured:
             g = torch.cuda.CUDAGraph()
