@@ -5,7 +5,8 @@
 //   static void compute(const P&, int i, int j, int cls, const T f[Q], T fo[Q]);  // bulk node
 //   static void finish(const P&, int i, int j, int cls, const T f[Q]);            // compute + store
 //   static double edge_bulk_node(const P&, int i, int j, int cls);  // edge node; returns rho
-//   static void stencil_node(...), boundary_close(...);               // curved-wall nodes
+//   static void wall_block<WAIT>(const P&, smem, int b);    // curved-wall nodes, 16 lanes each (WALL_LANES = 16), or
+//   static void stencil_node(...), boundary_close(...);    // 8 lanes, the closure in lane 0 (boundary_block)
 #pragma once
 #include <cuda_runtime.h>
 #include <algorithm>

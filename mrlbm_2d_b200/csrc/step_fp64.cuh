@@ -2,17 +2,14 @@
 //
 // One launch advances one time step of 2d_mrlbm.f90:231-535.  State between launches is
 // the post-collision population field fout (plus a ghost ring for populations the
-// reference never overwrites).  A launch has two kinds of blocks:
-//   * boundary blocks (the first nbblk): one thread per curved-wall boundary node.  Each
-//     pulls its own populations and those of its 8 bilinear-stencil nodes from the previous
-//     fout, recomputes the stencil moments, extrapolates velocity and rotated moments,
-//     runs the regularized closure, collides, stores, and computes the momentum-exchange
-//     force; forces and the inlet density sum are reduced with warp shuffles and the last
-//     boundary block to arrive writes one record per step.
-//   * bulk tiles: one thread per node and row of the tile; pull-stream, moments, edge
-//     Dirichlet values and regularized edge closures, moment-space collision, Hermite
-//     reconstruction, coalesced store.  Boundary nodes are skipped (the boundary blocks
-//     own them); solid nodes are ordinary nodes, as in the reference.
+// reference never overwrites).  Three kinds of work make a step up:
+//   * wall blocks: 16 lanes per curved-wall node (wall_block).  They pull the node's populations and
+//     those of its 8 bilinear-stencil nodes from the previous fout, recompute the stencil moments,
+//     extrapolate velocity and rotated moments, run the regularized closure, collide, store, and leave
+//     the momentum-exchange force of the node for the step's record;
+//   * edge blocks: one thread per domain-edge node, Dirichlet values and regularized edge closures;
+//   * bulk tiles: pull-stream, moments, moment-space collision, Hermite reconstruction, coalesced
+//     store.  Wall and edge nodes are skipped; solid nodes are ordinary nodes, as in the reference.
 // Every expression follows the reference's operation order (sums from k = 0 upwards,
 // products left to right); the translation unit is compiled with -fmad=false, so each
 // node's result is bit-identical to the reference's FP64 arithmetic.
