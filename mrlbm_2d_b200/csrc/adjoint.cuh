@@ -627,10 +627,25 @@ __device__ __forceinline__ void adjoint_wall(const P& p, const AdjArgs& a, int b
     const double kappa = (r == 0 ? G(G_T2) : -G(G_T3)) * ((s & 1) ? xd : 1.0 - xd) * ((s & 2) ? yd : 1.0 - yd);
     const double c = G(G_CTH), sn = G(G_STH), s2 = G(G_S2TH), c2 = G(G_C2TH), cc = G(G_CC), ss = G(G_SS);
     const double cxp = G(G_CXP + k), cyp = G(G_CYP + k), hxx = G(G_HXXP + k), hyy = G(G_HYYP + k), hxy = G(G_HXYP + k);
-    const double B11 = G(G_B11), B22 = G(G_B22), B12 = G(G_B12), F11 = G(G_F11), F22 = G(G_F22), F12 = G(G_F12);
     const double exk = ex(k), eyk = ey(k), Hx = exk != 0.0 ? (double)p.hp : (double)p.hm, Hy = eyk != 0.0 ? (double)p.hp : (double)p.hm;
     const double w = lane < Q ? (double)(k == 0 ? p.w[0] : k < 5 ? p.w[1] : p.w[5]) : 0.0;     // lanes past the directions add nothing
-    const double om = p.omega, om1 = p.omega1;
+    constexpr bool none = CL == CLOSURE_NONE, strong = CL == CLOSURE_STRONG, weak = CL == CLOSURE_WEAK;
+    const double om = p.omega, om1 = p.omega1;         // om1: the collision's, an FP32 handle's rounded to FP32
+    const double beta = strong ? 1.0 - om : 1.0;       // the closure's
+    // The closure's constant sums.  An FP32 handle's table has them rounded to FP32, and L11, L22 and L12 below take
+    // them from one another (which put gradients 1e-8 to 5e-8 of the largest entry off): there they are summed from the node's entries,
+    // like every other sum of the adjoint in FP64.
+    double B11 = 0.0, B22 = 0.0, B12 = 0.0, F11 = 0.0, F22 = 0.0, F12 = 0.0;
+    if constexpr (!none) {
+        if constexpr (sizeof(typename P::Real) == 8) {
+            B11 = G(G_B11); B22 = G(G_B22); B12 = G(G_B12);
+            F11 = G(G_F11); F22 = G(G_F22); F12 = G(G_F12);
+        } else {
+            const double b = 4.5 * w, sum = strong ? out : in;
+            B11 = sum16(sum * b * hxx); B22 = sum16(sum * b * hyy); B12 = sum16(sum * b * hxy);
+            F11 = sum16(in * b * hxx * hxy); F22 = sum16(in * b * hyy * hxy); F12 = sum16(in * b * hxy * hxy);
+        }
+    }
     wait_prior_grid();
 
     const int64_t own = p.L.at(i, j, k), src = p.L.at(i - ex(k), j - ey(k), k);     // wall nodes are interior nodes
@@ -657,7 +672,6 @@ __device__ __forceinline__ void adjoint_wall(const P& p, const AdjArgs& a, int b
     double X = sum16(half * kappa * xs), Y = sum16(half * kappa * ys);
     if (!p.mom_interp) X = Y = 0.0;
     // the node's own moments, where something of them survives
-    constexpr bool none = CL == CLOSURE_NONE;
     MacS<double> m0{1.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     double inv0 = 1.0;
     if (none || !p.vel_interp) {
@@ -673,8 +687,6 @@ __device__ __forceinline__ void adjoint_wall(const P& p, const AdjArgs& a, int b
     const double up = ux * c + uy * sn, vp = uy * c - ux * sn;
     double rho, mxx, myy, mxy;
     double A_p = 0.0, E_p = 0.0, rhoI = 1.0, mI = 0.0, D = 0.0, Z = 0.0, Pp = 0.0, den = 1.0, L11 = 0.0, L22 = 0.0, L12 = 1.0;
-    constexpr bool strong = CL == CLOSURE_STRONG, weak = CL == CLOSURE_WEAK;
-    const double beta = strong ? om1 : 1.0;
     if constexpr (none) {
         rho = m0.rho; mxx = m0.mxx; myy = m0.myy; mxy = m0.mxy;
     } else {
@@ -686,7 +698,7 @@ __device__ __forceinline__ void adjoint_wall(const P& p, const AdjArgs& a, int b
         if (strong || weak) A_p = sum16((strong ? out : in) * A);
         if (!weak) E_p = sum16((strong ? out : in) * E);
         if constexpr (strong || weak) {
-            Pp = strong ? om1 * A_p + om * E_p : A_p;
+            Pp = strong ? beta * A_p + om * E_p : A_p;
             L11 = beta * B11 * mI - F11;
             L22 = beta * B22 * mI - F22;
             L12 = 2.0 * (beta * B12 * mI - F12);
@@ -745,7 +757,7 @@ __device__ __forceinline__ void adjoint_wall(const P& p, const AdjArgs& a, int b
             mIb = -beta * t * (X * B11 + Y * B22 + 2.0 * Z * B12) - t * Pp;
             const double Pb = denb - t * mI;
             Db = t;
-            Ab = in * Db * hxy + (strong ? out * om1 * Pb : in * Pb);
+            Ab = in * Db * hxy + (strong ? out * beta * Pb : in * Pb);
             Eb = strong ? out * om * Pb : 0.0;
         } else {
             const double t = Zb / L12;
