@@ -67,11 +67,11 @@ __device__ __forceinline__ Dual operator+(Dual a, Dual b) { return Dual(a.v + b.
 __device__ __forceinline__ Dual operator-(Dual a, Dual b) { return Dual(a.v - b.v, a.d - b.d); }
 __device__ __forceinline__ Dual operator-(Dual a) { return Dual(-a.v, -a.d); }
 __device__ __forceinline__ Dual operator*(Dual a, Dual b) { return Dual(a.v * b.v, a.d * b.v + a.v * b.d); }
-// (one division each, a reciprocal: a division is some 40 instructions, and the edge nodes' maps divide
-// seven times in a row)
+// (one division each: a division is some 40 instructions, and the edge nodes' maps divide seven times in a
+// row.  The gradient over 400 steps of 512 x 128: 7.79 ms, with two divisions 8.11)
 __device__ __forceinline__ Dual operator/(Dual a, Dual b) {
-    const double r = 1.0 / b.v, q = a.v * r;
-    return Dual(q, (a.d - q * b.d) * r);
+    const double r = 1.0 / b.v, q = quotient(a.v, b.v, r);
+    return Dual(q, quotient(a.d - q * b.d, b.v, r));
 }
 __device__ __forceinline__ Dual operator+(Dual a, double b) { return Dual(a.v + b, a.d); }
 __device__ __forceinline__ Dual operator+(double a, Dual b) { return Dual(a + b.v, b.d); }
@@ -81,11 +81,11 @@ __device__ __forceinline__ Dual operator*(Dual a, double b) { return Dual(a.v * 
 __device__ __forceinline__ Dual operator*(double a, Dual b) { return Dual(a * b.v, a * b.d); }
 __device__ __forceinline__ Dual operator/(Dual a, double b) {
     const double r = 1.0 / b;
-    return Dual(a.v * r, a.d * r);
+    return Dual(quotient(a.v, b, r), quotient(a.d, b, r));
 }
 __device__ __forceinline__ Dual operator/(double a, Dual b) {
-    const double r = 1.0 / b.v, q = a * r;
-    return Dual(q, -q * b.d * r);
+    const double r = 1.0 / b.v, q = quotient(a, b.v, r);
+    return Dual(q, quotient(-q * b.d, b.v, r));
 }
 
 template <class S>
@@ -484,7 +484,7 @@ __device__ __forceinline__ void adjoint_bulk(const P& p, const AdjArgs& a, int t
 // Edge block b: 7 nodes of edge_node_ij x 18 threads, thread q of a node for its input q: own inputs
 // 0..8; at the outlet the copied neighbour's inputs 9..17; at the inlet q = 9 is u_in(j).  Every load
 // (the nodes' lambda^n, staged once and cleared for reuse, and each thread's inputs) is issued before
-// the first use: with the staging ahead of the gathers and two divisions per dual division these blocks
+// the first use: with the staging ahead of the gathers and two divisions per dual quotient these blocks
 // were the last of a step to end, 7.4 of its 8.4 us on 512 x 128 (the gradient over 400 steps 9.1 ms;
 // with this, and without the clearing of what adjoint_bulk stores outright, 8.1).
 template <class P>

@@ -65,3 +65,37 @@ def test_tile_division_magic_and_launch_counts(tmp_path):
     assert int(checked) > 10_000_000
     assert int(bad) == 0
     assert launches_ok == "1"
+
+
+QUOTIENT = r"""
+#include <cstdio>
+#include <cstdint>
+#include "adjoint.h"
+int main() {
+    long long plain = 0, bad = 0, n = 0;
+    uint64_t x = 88172645463325252ull;
+    auto draw = [&]() { x ^= x << 13; x ^= x >> 7; x ^= x << 17; return x; };
+    for (int t = 0; t < 2000000; ++t, ++n) {
+        const uint64_t u = draw(), v = draw();
+        const double a = std::ldexp(1.0 + (double)(u >> 12) * 0x1p-52, (int)(u % 64) - 32) * (u & 64 ? 1.0 : -1.0);
+        const double b = std::ldexp(1.0 + (double)(v >> 12) * 0x1p-52, (int)(v % 64) - 32);
+        if (a * (1.0 / b) != a / b) ++plain;
+        if (mrlbm::adj::quotient(a, b, 1.0 / b) != a / b) ++bad;
+    }
+    if (mrlbm::adj::quotient(0.0, 3.0, 1.0 / 3.0) != 0.0) ++bad;
+    std::printf("%lld %lld %lld\n", n, plain, bad);
+    return 0;
+}
+"""
+
+
+@pytest.mark.skipif(not os.path.isdir(CUDA_INC), reason="CUDA headers not installed")
+def test_adjoint_quotients_are_divisions(tmp_path):
+    """The dual numbers' quotients by a shared reciprocal round as the divisions they stand for."""
+    src, exe = tmp_path / "quotient.cpp", tmp_path / "quotient"
+    src.write_text(QUOTIENT)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-I", CSRC, "-I", os.path.join(ROOT, "include"), "-I",
+                    CUDA_INC, str(src), "-o", str(exe)], check=True)
+    n, plain, bad = (int(v) for v in subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split())
+    assert n == 2_000_000 and bad == 0
+    assert plain > n // 10                                    # the plain product would not do
