@@ -52,21 +52,33 @@ __device__ __forceinline__ bool is_interior(const StepParams<T>& p, int i, int j
     return col_interior(p, i) && j > 1 && j < p.L.ny;
 }
 
+// A value that an earlier launch may still be writing when this launch starts, read after the wait for it.
+// The read-only path (__ldg) is for data that nothing writes while the kernel runs, from its start on: its lines may
+// be copies from before the write.  This one reads the L2.
+template <class T>
+__device__ __forceinline__ T load_written(const T* q) { return __ldcg(q); }
+
+// f(i,j,:) of an interior node.
+template <class T>
+__device__ __forceinline__ void gather_written(const StepParams<T>& p, int i, int j, T f[Q]) {
+    const int pitch = p.L.pitch, plane = (int)p.L.plane;
+    const T* s = p.src + ((int)(j * pitch + i + p.L.off));
+#pragma unroll
+    for (int k = 0; k < Q; ++k) f[k] = load_written(s + (k * plane - ey(k) * pitch - ex(k)));
+}
+
 // f(i,j,:) of this step = fout of the previous step at the streaming sources
 // (stream_source in lattice.h).  Interior nodes take the branch-free fast path.
 template <class T>
 __device__ __forceinline__ void gather(const StepParams<T>& p, int i, int j, T f[Q]) {
     const int nx = p.L.nx, ny = p.L.ny;
-    const int pitch = p.L.pitch, plane = (int)p.L.plane;
     if (is_interior(p, i, j)) {
-        const T* s = p.src + ((int)(j * pitch + i + p.L.off));
-#pragma unroll
-        for (int k = 0; k < Q; ++k) f[k] = __ldg(s + (k * plane - ey(k) * pitch - ex(k)));
+        gather_written(p, i, j, f);
     } else {
 #pragma unroll
         for (int k = 0; k < Q; ++k) {
             SrcSlot sl = stream_source(nx, ny, i, j, k, p.xper, p.yper, p.freeslip, p.halo_l, p.halo_r);
-            f[k] = __ldg(p.src + p.L.at(sl.i, sl.j, sl.k));
+            f[k] = load_written(p.src + p.L.at(sl.i, sl.j, sl.k));
         }
         // overrides by a select over the nine slots: an index known only at run time would put
         // f in local memory, and each load would then wait for the one before to be stored
@@ -102,7 +114,7 @@ __device__ __forceinline__ void edge_gather(const StepParams<T>& p, int i, int j
             if (yhit && slip) o = reflected;
             if (yhit && p.yper) o = k * plane + (ey(k) > 0 ? ny - 1 : 1 - ny) * pitch;
         }
-        f[k] = __ldg(s + o);
+        f[k] = load_written(s + o);
     }
     for (int q = 0; q < p.n_ovr; ++q)                               // by a select over the nine, as in `gather`
         if (p.ovr[q].i == i && p.ovr[q].j == j) {
@@ -145,8 +157,10 @@ __device__ __forceinline__ void store_macro(const StepParams<T>& p, int i, int j
 // Field statistics: this step's post-closure u, v and p = rho cs2 (cs2 = 1/3, 2d_mrlbm.f90:153,
 // 237) added to FP64 running sums of x and x^2.  Explicit round-to-nearest operations keep the
 // sums free of contraction in every build, so they equal a host loop adding the same fields.
-// The six old sums of a node are loaded (read-only path; each slot belongs to one thread of
-// the launch) before the node's arithmetic, so their latency overlaps it.
+// The six old sums of a node are loaded before the node's arithmetic, so their latency overlaps it, and
+// from the L2: a slot belongs to one thread of a launch, its 32-byte sector does not.  In a pair
+// (step_pair.cuh) the first launch adds to the band's sums while the second's tiles read their neighbours',
+// and the second's other blocks read the band's afterwards.
 struct FieldPre { double v[6]; };
 
 template <class T>
@@ -154,7 +168,7 @@ __device__ __forceinline__ void fields_load(const StepParams<T>& p, int i, int j
     const int64_t n = (int64_t)(i - 1) + (int64_t)p.L.nx * (j - 1);
     const int64_t N = (int64_t)p.L.nx * p.L.ny;
 #pragma unroll
-    for (int c = 0; c < 6; ++c) q.v[c] = __ldg(p.fstat + n + c * N);
+    for (int c = 0; c < 6; ++c) q.v[c] = load_written(p.fstat + n + c * N);
 }
 
 // The sums after one more step's values, still in registers.

@@ -212,7 +212,7 @@ __device__ __forceinline__ Mac node_macro(const P& p, int i, int j, const double
 __device__ __forceinline__ void stencil_node(const P& p, int si, int sj, double cc, double ss, double s2, double& ux,
                                              double& uy, double& mx, double& my) {
     double f[Q];
-    gather_interior(p, si, sj, f);                  // stencil nodes are interior fluid nodes (checked at setup)
+    gather_written(p, si, sj, f);                   // stencil nodes are interior fluid nodes (checked at setup)
     const Mac m = moments(f, p.hm, p.hp);
     ux = m.ux;
     uy = m.uy;
@@ -331,7 +331,7 @@ __device__ __forceinline__ void wall_block(const P& p, unsigned char* smem, int 
     // the node's population of direction k (a wall node is an interior node)
     double fk = 0.0, ux = 0.0, uy = 0.0, mx = 0.0, my = 0.0;
     if (active) {
-        fk = __ldg(p.src + ((int64_t)k * p.L.plane + (int64_t)(nj - eky) * p.L.pitch + (ni - ekx) + p.L.off));
+        fk = load_written(p.src + ((int64_t)k * p.L.plane + (int64_t)(nj - eky) * p.L.pitch + (ni - ekx) + p.L.off));
         if (interp) {
             stencil_node(p, si, sj, cc, ss, s2, ux, uy, mx, my);
             const double wx = (s & 1) ? xd : (1.0 - xd);

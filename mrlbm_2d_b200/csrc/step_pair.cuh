@@ -62,7 +62,7 @@ __device__ __forceinline__ void band_node(const typename Phys::P& p, const PairB
     if (cls == CLS_SOLID && p.call && p.plot_every > 0 && (__ldg(p.call) + p.bstep + 1) % p.plot_every == 0)
         cls = CLS_SOLID_ZERO;
     typename Phys::T f[Q];
-    gather_interior(p, i, j, f);
+    gather_written(p, i, j, f);                                  // at the second level the other launch wrote it
     if (FIRST && p.fstat && i > 2 && i < nx - 1 && j > 2 && j < ny - 1 &&
         !(i >= core.x0 && i <= core.x1 && j >= core.y0 && j <= core.y1)) {
         typename Phys::P nosum = p;
