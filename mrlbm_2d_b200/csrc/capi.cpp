@@ -107,6 +107,7 @@ struct mrlbm_handle {
     uint64_t replay_clock = 0;
     int64_t stepped = 0;                      // steps taken by the handle, the autotuner's left out
     bool no_replay = false;                   // autotuner trials of single shapes
+    bool replay_failed = false;               // a run could not be captured or launched: launched steps from then on
     int* d_call = nullptr;                    // call state of the replay (StepParams::call)
     std::vector<OvrEntry> ovr;                // loaded-state overrides (see OvrEntry)
     bool ovr_live = false;                    // true until the first step after a load
@@ -670,7 +671,7 @@ constexpr int REPLAY_AFTER = 24;
 // Length of the run to replay for the next `left` steps, or 0: launched steps.  Every step of the run must be
 // one whose launch differs from its captured form in the call state only.
 int replay_length(const mrlbm_handle* h, int left) {
-    if (left < REPLAY_STEPS[1] || h->no_replay || h->ovr_live || h->surf_on || !h->own_stream || is_tma_cfg(h->tile_cfg) ||
+    if (left < REPLAY_STEPS[1] || h->no_replay || h->replay_failed || h->ovr_live || h->surf_on || !h->own_stream || is_tma_cfg(h->tile_cfg) ||
         (int64_t)h->L.nx * h->L.ny > REPLAY_MAX_NODES || h->halo_l || h->halo_r)
         return 0;
     const mrlbm_config& c = h->cfg;
@@ -734,8 +735,9 @@ int capture_run(mrlbm_handle* h, int n, bool fields, cudaStream_t st) {
     return 0;
 }
 
-// The graph of n steps from the handle's current level (captured on the handle's own stream if none is kept).
-int replay_graph(mrlbm_handle* h, int n, bool fields, mrlbm_handle::Replay*& out) {
+// The graph of n steps from the handle's current level (captured on the handle's own stream if none is kept), or
+// null when it cannot be made.
+mrlbm_handle::Replay* replay_graph(mrlbm_handle* h, int n, bool fields) {
     const bool fp64 = h->precision == MRLBM_FP64;
     const std::vector<uintptr_t> sig = {(uintptr_t)h->cur, (uintptr_t)h->tile_cfg, (uintptr_t)h->pairs, (uintptr_t)h->mid,
                                         h->has_uin ? (uintptr_t)h->d_uin : 0, h->has_body ? (uintptr_t)h->d_body : 0,
@@ -744,35 +746,34 @@ int replay_graph(mrlbm_handle* h, int n, bool fields, mrlbm_handle::Replay*& out
     for (auto& q : h->replay) {
         if (q.exec && q.steps == n && q.sig == sig) {
             q.used = ++h->replay_clock;
-            out = &q;
-            return MRLBM_OK;
+            return &q;
         }
         if (q.used < g->used) g = &q;                              // least recently used
     }
-    if (!h->d_call) CK(cudaMalloc((void**)&h->d_call, 5 * sizeof(int)));
+    if (!h->d_call && cudaMalloc((void**)&h->d_call, 5 * sizeof(int)) != cudaSuccess) {
+        h->d_call = nullptr;
+        return nullptr;
+    }
     if (g->exec) {
-        CK(cudaStreamSynchronize(h->stream));
+        if (cudaStreamSynchronize(h->stream) != cudaSuccess) return nullptr;
         cudaGraphExecDestroy(g->exec);
         *g = mrlbm_handle::Replay{};
     }
-    CK(cudaStreamBeginCapture(h->own_stream, cudaStreamCaptureModeThreadLocal));
+    if (cudaStreamBeginCapture(h->own_stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) return nullptr;
     const int rc = fp64 ? capture_run<double>(h, n, fields, h->own_stream) : capture_run<float>(h, n, fields, h->own_stream);
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(h->own_stream, &graph);
     if (rc == 0 && e == cudaSuccess) e = cudaGraphInstantiate(&g->exec, graph, 0);
     if (graph) cudaGraphDestroy(graph);
     if (rc != 0 || e != cudaSuccess) {
-        cudaGetLastError();
         g->exec = nullptr;
-        if (rc == -2) return fail(h, MRLBM_EUNSUPPORTED, "tile shape does not fit this precision");
-        return fail(h, MRLBM_ECUDA, "capturing a run of steps failed");
+        return nullptr;
     }
     g->steps = n;
     g->sig = sig;
     g->launches = h->pairs ? n / 2 * PAIR_LAUNCHES : n * step_launches(!fp64, h->tile_cfg);
     g->used = ++h->replay_clock;
-    out = g;
-    return MRLBM_OK;
+    return g;
 }
 
 // This thread's calls as they would be were no other thread capturing: a graph being captured elsewhere in
@@ -783,18 +784,22 @@ struct RelaxedCapture {
     ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
 
-int step_replay(mrlbm_handle* h, int n) {
+// Replays n steps.  False, and nothing has changed, when the graph, its call state or its launch could not be
+// had (memory, most likely): the caller launches the steps, and reports an error that stays.
+bool step_replay(mrlbm_handle* h, int n) {
     RelaxedCapture relaxed;
     const int z = h->iter + n;
     const bool fields = fields_at(h, h->iter + 1);
-    mrlbm_handle::Replay* g = nullptr;
-    const int rc = replay_graph(h, n, fields, g);
-    if (rc != MRLBM_OK) return rc;
+    mrlbm_handle::Replay* g = replay_graph(h, n, fields);
     // (pageable memory: the copy takes the words before it returns)
     const int call[5] = {h->iter, h->ring_n, h->pend.on ? h->pend.iter : 0, h->pend.on ? h->pend.rec_idx : -1,
                          h->pend.on ? h->pend.slot : 0};
-    CK(cudaMemcpyAsync(h->d_call, call, sizeof call, cudaMemcpyHostToDevice, h->stream));
-    CK(cudaGraphLaunch(g->exec, h->stream));
+    if (!g || cudaMemcpyAsync(h->d_call, call, sizeof call, cudaMemcpyHostToDevice, h->stream) != cudaSuccess ||
+        cudaGraphLaunch(g->exec, h->stream) != cudaSuccess) {
+        cudaGetLastError();
+        h->replay_failed = true;
+        return false;
+    }
     h->launches += g->launches;
     const int lo = std::max(h->iter + 1, h->cfg.statsbegin), hi = std::min(z, h->cfg.statsend);
     if (h->cfg.post_process && hi >= lo) h->ring_n += hi - lo + 1;
@@ -803,7 +808,7 @@ int step_replay(mrlbm_handle* h, int n) {
     if (fields) h->fstat_n += n;
     h->iter = z;
     h->cur ^= (h->pairs ? n / 2 : n) & 1;
-    return MRLBM_OK;
+    return true;
 }
 
 void free_all(mrlbm_handle* h) {
@@ -1501,9 +1506,7 @@ int mrlbm_step(mrlbm_handle* h, int32_t nsteps, int32_t flags) {
         // a step with macroscopic output is taken alone
         const int s0 = s;
         const int run = replay_length(h, nsteps - s - ((flags & MRLBM_STEP_MACRO) ? 1 : 0));
-        if (run > 0) {
-            rc = step_replay(h, run);
-            if (rc != MRLBM_OK) return rc;
+        if (run > 0 && step_replay(h, run)) {
             s += run;
         } else if (nsteps - s >= ((flags & MRLBM_STEP_MACRO) ? 3 : 2) && pair_ok(h)) {
             rc = launch_two(h);
@@ -1642,6 +1645,7 @@ int mrlbm_step_noalloc(mrlbm_handle* h, void* d_state, const double* d_f0, int32
 int mrlbm_set_tile_config(mrlbm_handle* h, int32_t cfg) {
     if (!h || cfg < 0 || cfg >= N_ALL_CFGS) return MRLBM_EINVAL;
     h->tile_cfg = cfg;
+    h->replay_failed = false;                           // another shape, another capture
     return MRLBM_OK;
 }
 
