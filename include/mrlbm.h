@@ -163,7 +163,8 @@ int mrlbm_set_inlet_profile(mrlbm_handle* h, const double* u_in);
  * macroscopic fields for mrlbm_get_macro. */
 /* On large lattices a call takes its steps two at a time (each pair reads and writes the
  * populations once; the same bits as two single steps), a last odd step and a step with macroscopic output
- * alone.  Pairs need a third population level on the device; without the memory for it, and on
+ * alone.  Pairs need a third population level on the device, taken if it is at most a quarter of the
+ * free memory and given back when a later call of the handle finds none left; without it, and on
  * x-slabs, steps are single.  The rule is by size and precision, mrlbm_autotune replaces it by a
  * measurement, and MRLBM_PAIRS=0 or 1 in the environment at creation replaces both. */
 #define MRLBM_STEP_MACRO   1

@@ -52,6 +52,8 @@ struct mrlbm_handle {
     // steps taken in pairs (step_pair.cuh): the buffer of the intermediate level's band
     bool pairs = false, pairs_fixed = false;  // fixed: by the environment, not by rule or autotuner
     void* mid = nullptr;
+    bool paired() const { return pairs && mid; }
+    const std::vector<mrlbm_handle*>* mates = nullptr;   // the cases of the batch that owns the handle
     PairPlan plan{};
     CUtensorMap tmap_pair[2];                 // 3-D maps (columns, rows, planes) of both time levels
     void* d_bgeo = nullptr;
@@ -214,11 +216,38 @@ std::vector<OvrEntry> slot_conflicts(const mrlbm_handle* h) {
     return out;
 }
 
+void disable_pairs(mrlbm_handle* h) {
+    h->pairs = false;
+    if (h->mid) cudaFree(h->mid);
+    h->mid = nullptr;
+}
+
+// Device memory for a handle.  When there is none left, the pairs' band (a third level that only makes steps
+// faster) goes back first, of every case of a batch.
+cudaError_t device_alloc(mrlbm_handle* h, void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        bool freed = h->mid != nullptr;
+        disable_pairs(h);
+        if (h->mates)
+            for (mrlbm_handle* m : *h->mates) {
+                freed = freed || m->mid;
+                disable_pairs(m);
+            }
+        if (freed) {
+            cudaGetLastError();
+            e = cudaMalloc(p, bytes);
+        }
+    }
+    if (e != cudaSuccess) *p = nullptr;
+    return e;
+}
+
 // f(nx,ny,0:8) on the host -> both padded time levels: one host->device copy and a scatter
 // kernel (state_io.cu).
 int upload_state(mrlbm_handle* h, const double* f) {
     const size_t n = (size_t)h->L.nx * h->L.ny * Q;
-    if (!h->d_fstage) CK(cudaMalloc((void**)&h->d_fstage, n * sizeof(double)));
+    if (!h->d_fstage) CK(device_alloc(h, (void**)&h->d_fstage, n * sizeof(double)));
     CK(cudaMemcpyAsync(h->d_fstage, f, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     const mrlbm_config& c = h->cfg;
     CK(launch_scatter_state(h->precision, h->d_fstage, h->buf[0], h->buf[1], h->L, c.x_periodic != 0,
@@ -233,7 +262,7 @@ int upload_state(mrlbm_handle* h, const double* f) {
         e.v = h->precision == MRLBM_FP64 ? v : (double)(float)(v - h->lat.w[e.k]);
     }
     if (!h->ovr.empty()) {                // at most the 4 x 9 corner slots; allocated once
-        if (!h->d_ovr) CK(cudaMalloc((void**)&h->d_ovr, 4 * Q * sizeof(OvrEntry)));
+        if (!h->d_ovr) CK(device_alloc(h, (void**)&h->d_ovr, 4 * Q * sizeof(OvrEntry)));
         CK(cudaMemcpyAsync(h->d_ovr, h->ovr.data(), h->ovr.size() * sizeof(OvrEntry), cudaMemcpyHostToDevice,
                            h->stream));
     }
@@ -340,7 +369,7 @@ int prepare_tma(mrlbm_handle* h, int cfg) {
     }
     if (per_sm == 0) return fail(h, MRLBM_EUNSUPPORTED, "TMA shape does not fit this precision");
     if (!h->d_tile_ctr) {
-        CK(cudaMalloc((void**)&h->d_tile_ctr, sizeof(unsigned long long)));
+        CK(device_alloc(h, (void**)&h->d_tile_ctr, sizeof(unsigned long long)));
         CK(cudaMemsetAsync(h->d_tile_ctr, 0, sizeof(unsigned long long), h->stream));
         h->tile_base = 0;
     }
@@ -548,9 +577,10 @@ void make_pair_plan(mrlbm_handle* h, int sharers) {
     q.chunks = pair_chunks(h->L.nx, h->L.ny, h->elem == 8 ? PAIR_STRIPS64 : PAIR_STRIPS32, std::max(1, PAIR_MINB * h->num_sms / sharers));
 }
 
-// `sharers`: cases that step on the GPU at the same time (a batch), each with its part of the resident blocks.
 // Take steps in pairs from now on: the band buffer, with the ghost ring every level carries.
-// False (and single steps as before) when there is no memory for it.
+// False (and single steps as before) when there is no memory to spare for it: it takes at most a quarter of what is
+// free, since a program that fills the GPU with other things still has to find the room it found before.
+// `sharers`: cases that step on the GPU at the same time (a batch), each with its part of the resident blocks.
 bool enable_pairs(mrlbm_handle* h, int sharers = 1) {
     if (!pairs_possible(h)) return false;
     if (!h->mid) {
@@ -565,22 +595,21 @@ bool enable_pairs(mrlbm_handle* h, int sharers = 1) {
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
                 return false;
         }
-        if (cudaMalloc(&h->mid, (size_t)h->L.total() * h->elem) != cudaSuccess) {
+        const size_t bytes = (size_t)h->L.total() * h->elem;
+        size_t free_now = 0, total = 0;
+        if (cudaMemGetInfo(&free_now, &total) != cudaSuccess || bytes > free_now / 4 || cudaMalloc(&h->mid, bytes) != cudaSuccess) {
             cudaGetLastError();
             h->mid = nullptr;
             return false;
         }
-        if (launch_copy_ring(h->precision, h->buf[h->cur], h->mid, h->L, h->stream) != cudaSuccess) return false;
+        if (launch_copy_ring(h->precision, h->buf[h->cur], h->mid, h->L, h->stream) != cudaSuccess) {
+            disable_pairs(h);
+            return false;
+        }
     }
     make_pair_plan(h, sharers);
     h->pairs = true;
     return true;
-}
-
-void disable_pairs(mrlbm_handle* h) {
-    h->pairs = false;
-    if (h->mid) cudaFree(h->mid);
-    h->mid = nullptr;
 }
 
 bool stats_at(const mrlbm_handle* h, int iter) {
@@ -597,7 +626,7 @@ bool fields_at(const mrlbm_handle* h, int iter) { return h->d_fstat && iter >= h
 // A TMA shape newly set is taken by a single step first, which refuses those that do not fit the precision.
 bool pair_ok(const mrlbm_handle* h) {
     const int a = h->iter + 1, b = h->iter + 2;
-    return h->pairs && (!is_tma_cfg(h->tile_cfg) || h->tmap_cfg == h->tile_cfg) && !h->ovr_live &&
+    return h->paired() && (!is_tma_cfg(h->tile_cfg) || h->tmap_cfg == h->tile_cfg) && !h->ovr_live &&
            h->ring_n + 2 <= RING_CAP && fields_at(h, a) == fields_at(h, b) && !(h->surf_on && (stats_at(h, a) || stats_at(h, b)));
 }
 
@@ -717,7 +746,7 @@ int capture_run(mrlbm_handle* h, int n, bool fields, cudaStream_t st) {
     };
     for (int s = 0; s < n;) {
         int rc;
-        if (h->pairs) {
+        if (h->paired()) {
             StepParams<T> p[2] = {params(s), params(s + 1)};
             rc = launch_pair_params<T>(h, cur, p, st);
             s += 2;
@@ -739,7 +768,7 @@ int capture_run(mrlbm_handle* h, int n, bool fields, cudaStream_t st) {
 // null when it cannot be made.
 mrlbm_handle::Replay* replay_graph(mrlbm_handle* h, int n, bool fields) {
     const bool fp64 = h->precision == MRLBM_FP64;
-    const std::vector<uintptr_t> sig = {(uintptr_t)h->cur, (uintptr_t)h->tile_cfg, (uintptr_t)h->pairs, (uintptr_t)h->mid,
+    const std::vector<uintptr_t> sig = {(uintptr_t)h->cur, (uintptr_t)h->tile_cfg, (uintptr_t)h->paired(), (uintptr_t)h->mid,
                                         h->has_uin ? (uintptr_t)h->d_uin : 0, h->has_body ? (uintptr_t)h->d_body : 0,
                                         fields ? (uintptr_t)h->d_fstat : 0};
     mrlbm_handle::Replay* g = &h->replay[0];
@@ -771,7 +800,7 @@ mrlbm_handle::Replay* replay_graph(mrlbm_handle* h, int n, bool fields) {
     }
     g->steps = n;
     g->sig = sig;
-    g->launches = h->pairs ? n / 2 * PAIR_LAUNCHES : n * step_launches(!fp64, h->tile_cfg);
+    g->launches = h->paired() ? n / 2 * PAIR_LAUNCHES : n * step_launches(!fp64, h->tile_cfg);
     g->used = ++h->replay_clock;
     return g;
 }
@@ -807,7 +836,7 @@ bool step_replay(mrlbm_handle* h, int n) {
     if (h->pend.on) h->pend = mrlbm_handle::Pending{true, 2 + ((n - 1) & 1), h->ring_n - 1, z};
     if (fields) h->fstat_n += n;
     h->iter = z;
-    h->cur ^= (h->pairs ? n / 2 : n) & 1;
+    h->cur ^= (h->paired() ? n / 2 : n) & 1;
     return true;
 }
 
@@ -907,7 +936,8 @@ int mrlbm_config_resolve_geometry(mrlbm_config* cfg) {
     return MRLBM_OK;
 }
 
-static int create_impl(const mrlbm_config* cfg, int precision, int device, int sx0, int sx1, mrlbm_handle** out) {
+// `alone`: not a case of a batch, which decides on pairs for all of its cases.
+static int create_impl(const mrlbm_config* cfg, int precision, int device, int sx0, int sx1, bool alone, mrlbm_handle** out) {
     if (!cfg || !out) return MRLBM_EINVAL;
     *out = nullptr;
     if (precision != MRLBM_FP64 && precision != MRLBM_FP32) {
@@ -1039,19 +1069,19 @@ static int create_impl(const mrlbm_config* cfg, int precision, int device, int s
     h->iter = 1;
     const char* pv = std::getenv("MRLBM_PAIRS");
     h->pairs_fixed = pv != nullptr;
-    if (pv ? std::atoi(pv) != 0 : pairs_pay(h)) enable_pairs(h);
+    if (alone && (pv ? std::atoi(pv) != 0 : pairs_pay(h))) enable_pairs(h);
     *out = h;
     return MRLBM_OK;
 }
 
 int mrlbm_create(const mrlbm_config* cfg, int precision, int device, mrlbm_handle** out) {
-    return create_impl(cfg, precision, device, 0, 0, out);
+    return create_impl(cfg, precision, device, 0, 0, true, out);
 }
 
 int mrlbm_create_slab(const mrlbm_config* cfg, int precision, int device, int32_t gx0, int32_t gx1,
                       mrlbm_handle** out) {
     if (gx0 < 1) return MRLBM_EINVAL;
-    return create_impl(cfg, precision, device, gx0, gx1, out);
+    return create_impl(cfg, precision, device, gx0, gx1, true, out);
 }
 
 // Halo columns: side 0 is the left face (the populations moving left, k = 3, 6, 7, of column 1
@@ -1330,7 +1360,7 @@ int mrlbm_get_state(mrlbm_handle* h, double* f) {
     CK(cudaSetDevice(h->device));
     const int nx = h->L.nx, ny = h->L.ny;
     const size_t N = (size_t)nx * ny;
-    if (!h->d_fstage) CK(cudaMalloc((void**)&h->d_fstage, N * Q * sizeof(double)));
+    if (!h->d_fstage) CK(device_alloc(h, (void**)&h->d_fstage, N * Q * sizeof(double)));
     const mrlbm_config& c = h->cfg;
     CK(launch_gather_state(h->precision, h->buf[h->cur], h->d_fstage, h->L, c.x_periodic != 0, c.y_periodic != 0,
                            c.wall_mode == MRLBM_WALL_FREESLIP && !c.y_periodic, h->lat.w, h->stream, h->halo_l, h->halo_r));
@@ -1350,7 +1380,7 @@ int mrlbm_set_inlet_profile(mrlbm_handle* h, const double* u_in) {
     CK(cudaSetDevice(h->device));
     if (!u_in) { h->has_uin = false; return MRLBM_OK; }
     const int ny = h->L.ny;
-    if (!h->d_uin) CK(cudaMalloc((void**)&h->d_uin, (size_t)ny * sizeof(double)));
+    if (!h->d_uin) CK(device_alloc(h, (void**)&h->d_uin, (size_t)ny * sizeof(double)));
     if (h->precision == MRLBM_FP64) {
         CK(cudaMemcpyAsync(h->d_uin, u_in, (size_t)ny * 8, cudaMemcpyHostToDevice, h->stream));
     } else {
@@ -1423,12 +1453,12 @@ int mrlbm_surface_enable(mrlbm_handle* h, int32_t enable) {
             sumw[i] = sw;
         }
         h->surf_cap = (int)std::max<size_t>(1, std::min<size_t>(RING_CAP, ((size_t)64 << 20) / ((size_t)2 * nb * sizeof(double))));
-        CK(cudaMalloc((void**)&h->d_quad, quad.size() * sizeof(double)));
-        CK(cudaMalloc((void**)&h->d_sidx, nb * sizeof(int)));
-        CK(cudaMalloc((void**)&h->d_W, W.size() * sizeof(double)));
-        CK(cudaMalloc((void**)&h->d_sumw, nb * sizeof(double)));
-        CK(cudaMalloc((void**)&h->d_sring, (size_t)h->surf_cap * 2 * nb * sizeof(double)));
-        CK(cudaMalloc((void**)&h->d_pring, (size_t)h->surf_cap * 12 * sizeof(double)));
+        CK(device_alloc(h, (void**)&h->d_quad, quad.size() * sizeof(double)));
+        CK(device_alloc(h, (void**)&h->d_sidx, nb * sizeof(int)));
+        CK(device_alloc(h, (void**)&h->d_W, W.size() * sizeof(double)));
+        CK(device_alloc(h, (void**)&h->d_sumw, nb * sizeof(double)));
+        CK(device_alloc(h, (void**)&h->d_sring, (size_t)h->surf_cap * 2 * nb * sizeof(double)));
+        CK(device_alloc(h, (void**)&h->d_pring, (size_t)h->surf_cap * 12 * sizeof(double)));
         CK(cudaMemcpyAsync(h->d_quad, quad.data(), quad.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
         std::vector<int> place(nb);
         for (int i = 0; i < nb; ++i) place[idx[i]] = i;
@@ -1482,7 +1512,7 @@ int mrlbm_set_body_force(mrlbm_handle* h, const double* g) {
     CK(cudaSetDevice(h->device));
     if (!g) { h->has_body = false; return MRLBM_OK; }
     const size_t n2 = (size_t)2 * h->L.nx * h->L.ny;
-    if (!h->d_body) CK(cudaMalloc(&h->d_body, n2 * h->elem));
+    if (!h->d_body) CK(device_alloc(h, &h->d_body, n2 * h->elem));
     if (h->precision == MRLBM_FP64) {
         CK(cudaMemcpyAsync(h->d_body, g, n2 * 8, cudaMemcpyHostToDevice, h->stream));
         CK(cudaStreamSynchronize(h->stream));
@@ -1500,7 +1530,7 @@ int mrlbm_step(mrlbm_handle* h, int32_t nsteps, int32_t flags) {
     if (h->host_only) return fail(h, MRLBM_ENODEVICE, "host-only handle (created with device -1)");
     CK(cudaSetDevice(h->device));
     if ((flags & MRLBM_STEP_MACRO) && !h->d_macro)
-        CK(cudaMalloc((void**)&h->d_macro, (size_t)6 * h->L.nx * h->L.ny * sizeof(double)));
+        CK(device_alloc(h, (void**)&h->d_macro, (size_t)6 * h->L.nx * h->L.ny * sizeof(double)));
     for (int s = 0; s < nsteps;) {
         int rc;
         // a step with macroscopic output is taken alone
@@ -1543,8 +1573,8 @@ int mrlbm_field_stats_window(mrlbm_handle* h, int32_t begin_iter, int32_t end_it
     CK(cudaSetDevice(h->device));
     const size_t bytes = (size_t)6 * h->L.nx * h->L.ny * sizeof(double);
     if (!h->d_fstat) {
-        CK(cudaMalloc((void**)&h->d_fstat, bytes));
-        CK(cudaMalloc((void**)&h->d_fstat_out, bytes));
+        CK(device_alloc(h, (void**)&h->d_fstat, bytes));
+        CK(device_alloc(h, (void**)&h->d_fstat_out, bytes));
     }
     CK(cudaMemsetAsync(h->d_fstat, 0, bytes, h->stream));
     h->fstat_begin = begin_iter;
@@ -1664,8 +1694,8 @@ int mrlbm_autotune(mrlbm_handle* h, int32_t trial_steps, int32_t* best_cfg, doub
     // everything a trial changes is saved and put back: both time levels, iteration, ring
     const size_t bytes = (size_t)h->L.total() * h->elem;
     void* save[2] = {nullptr, nullptr};
-    CK(cudaMalloc(&save[0], bytes));
-    if (cudaMalloc(&save[1], bytes) != cudaSuccess) {
+    CK(device_alloc(h, &save[0], bytes));
+    if (device_alloc(h, &save[1], bytes) != cudaSuccess) {
         cudaFree(save[0]);
         return fail(h, MRLBM_ECUDA, "cudaMalloc autotune save");
     }
@@ -1682,7 +1712,7 @@ int mrlbm_autotune(mrlbm_handle* h, int32_t trial_steps, int32_t* best_cfg, doub
     double* fsave = nullptr;
     h->surf_on = false;
     if (h->d_fstat) {
-        if (cudaMalloc((void**)&fsave, fbytes) != cudaSuccess ||
+        if (device_alloc(h, (void**)&fsave, fbytes) != cudaSuccess ||
             cudaMemcpyAsync(fsave, h->d_fstat, fbytes, cudaMemcpyDeviceToDevice, h->stream) != cudaSuccess) {
             if (fsave) cudaFree(fsave);
             fsave = nullptr;
@@ -1869,7 +1899,7 @@ extern "C" int mrlbm_adjoint_drag(mrlbm_handle* h, int32_t nsteps, int32_t windo
         if (h->adj_ws) cudaFree(h->adj_ws);
         h->adj_ws = nullptr;
         h->adj_ws_bytes = 0;
-        if (cudaMalloc(&h->adj_ws, ws) != cudaSuccess) {
+        if (device_alloc(h, &h->adj_ws, ws) != cudaSuccess) {
             cudaGetLastError();
             return fail(h, MRLBM_ECUDA, "adjoint: device memory for checkpoints and adjoint fields");
         }
@@ -2217,10 +2247,11 @@ int batch_call_streams(mrlbm_batch* b, int steps) {
         }
         BCK(cudaEventCreateWithFlags(&b->fork_ev, cudaEventDisableTiming));
         BCK(cudaEventCreateWithFlags(&b->call_staged, cudaEventDisableTiming));
-        BCK(cudaMalloc((void**)&b->d_call, sizeof(int) * 2 * n));
+        BCK(device_alloc(b->h[0], (void**)&b->d_call, sizeof(int) * 2 * n));
         BCK(cudaMallocHost((void**)&b->h_call, sizeof(int) * 2 * n));
         BCK(cudaEventRecord(b->call_staged, b->stream));
     }
+    for (mrlbm_handle* h : b->h) b->pairs = b->pairs && h->mid;   // (a case's memory ran short: device_alloc)
     for (mrlbm_handle* h : b->h) {
         int rc = finish_pending(h);
         if (rc == MRLBM_OK && h->ring_n + stats_in(h->cfg, h->iter + 1, h->iter + steps) > RING_CAP) rc = drain_ring(h);
@@ -2303,7 +2334,7 @@ int batch_call(mrlbm_batch* b, int steps, int want_macro) {
             if (rc != MRLBM_OK) return bfail(b, rc, h->err);
         }
         if (want_macro && !h->d_macro)
-            BCK(cudaMalloc((void**)&h->d_macro, (size_t)6 * h->L.nx * h->L.ny * sizeof(double)));
+            BCK(device_alloc(h, (void**)&h->d_macro, (size_t)6 * h->L.nx * h->L.ny * sizeof(double)));
     }
     // stage the per-call parameters in pinned memory and upload them
     const int si = b->stage_i;
@@ -2331,7 +2362,7 @@ int batch_call(mrlbm_batch* b, int steps, int want_macro) {
             if (b->d_item_case) cudaFree(b->d_item_case);
             b->d_item_case = nullptr;
             b->item_case_cap = 0;
-            BCK(cudaMalloc((void**)&b->d_item_case, sizeof(int) * (size_t)items));
+            BCK(device_alloc(b->h[0], (void**)&b->d_item_case, sizeof(int) * (size_t)items));
             b->item_case_cap = (size_t)items;
         }
         BCK(cudaMemcpy(b->d_item_case, tab.data(), sizeof(int) * (size_t)items, cudaMemcpyHostToDevice));
@@ -2480,7 +2511,7 @@ int mrlbm_batch_create(const mrlbm_config* cfgs, int32_t ncases, int precision, 
     cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, device);
     for (int c = 0; c < ncases; ++c) {
         mrlbm_handle* h = nullptr;
-        int rc = mrlbm_create(cfgs + c, precision, device, &h);
+        int rc = create_impl(cfgs + c, precision, device, 0, 0, false, &h);
         if (rc != MRLBM_OK) return bail(rc, "case " + std::to_string(c) + ": " + g_create_error);
         b->h.push_back(h);
         if (h->own_stream) {
@@ -2489,18 +2520,20 @@ int mrlbm_batch_create(const mrlbm_config* cfgs, int32_t ncases, int precision, 
             h->own_stream = nullptr;
         }
         h->stream = b->stream;
-        b->pairs_fixed = b->pairs_fixed || h->pairs_fixed;
-        b->pairs = (c == 0 || b->pairs) && h->pairs && h->pairs_fixed;
     }
-    if (b->pairs)
-        for (mrlbm_handle* h : b->h) enable_pairs(h, ncases);
-    else
-        for (mrlbm_handle* h : b->h) disable_pairs(h);  // one step at a time until the autotuner finds otherwise
+    // one step at a time until the autotuner finds otherwise, or as MRLBM_PAIRS says
+    for (mrlbm_handle* h : b->h) h->mates = &b->h;
+    const char* pv = std::getenv("MRLBM_PAIRS");
+    b->pairs_fixed = pv != nullptr;
+    b->pairs = pv && std::atoi(pv) != 0;
+    for (mrlbm_handle* h : b->h) b->pairs = b->pairs && enable_pairs(h, ncases);
+    if (!b->pairs)
+        for (mrlbm_handle* h : b->h) disable_pairs(h);
     b->stage_bytes = batch_param_bytes(b);
-    bool ok = cudaMalloc(&b->d_params, b->stage_bytes) == cudaSuccess &&
-              cudaMalloc((void**)&b->d_cases, sizeof(BatchCase) * ncases) == cudaSuccess &&
-              cudaMalloc((void**)&b->d_off, sizeof(int) * (2 * ncases + 2)) == cudaSuccess &&
-              cudaMalloc((void**)&b->d_bar, sizeof(BatchBarrier)) == cudaSuccess &&
+    bool ok = device_alloc(b->h[0], &b->d_params, b->stage_bytes) == cudaSuccess &&
+              device_alloc(b->h[0], (void**)&b->d_cases, sizeof(BatchCase) * ncases) == cudaSuccess &&
+              device_alloc(b->h[0], (void**)&b->d_off, sizeof(int) * (2 * ncases + 2)) == cudaSuccess &&
+              device_alloc(b->h[0], (void**)&b->d_bar, sizeof(BatchBarrier)) == cudaSuccess &&
               cudaMemsetAsync(b->d_bar, 0, sizeof(BatchBarrier), b->stream) == cudaSuccess;
     for (int i = 0; ok && i < 2; ++i)
         ok = cudaMallocHost((void**)&b->h_stage[i], b->stage_bytes) == cudaSuccess &&
@@ -2619,12 +2652,12 @@ int mrlbm_batch_autotune(mrlbm_batch* b, int32_t trial_steps, double* best_ms_pe
         s = Saved{{nullptr, nullptr}, nullptr, h->iter, h->cur, h->ring_n, h->ovr_live, h->fstat_n, h->hist.size()};
         const size_t bytes = (size_t)h->L.total() * h->elem;
         for (int k = 0; k < 2; ++k) {
-            BCK(cudaMalloc(&s.buf[k], bytes));
+            BCK(device_alloc(h, &s.buf[k], bytes));
             BCK(cudaMemcpyAsync(s.buf[k], h->buf[k], bytes, cudaMemcpyDeviceToDevice, b->stream));
         }
         if (h->d_fstat) {
             const size_t fb = (size_t)6 * h->L.nx * h->L.ny * sizeof(double);
-            BCK(cudaMalloc((void**)&s.fstat, fb));
+            BCK(device_alloc(h, (void**)&s.fstat, fb));
             BCK(cudaMemcpyAsync(s.fstat, h->d_fstat, fb, cudaMemcpyDeviceToDevice, b->stream));
         }
     }

@@ -76,6 +76,7 @@ void fake_reset() {
     dangling = captures = 0;
 }
 void fake_fail(const char* call, int times) { failing[call] = times; }
+void fake_mark() { peak = used; }
 void fake_limit(int64_t bytes) { limit = (size_t)bytes; }
 int64_t fake_used() { return (int64_t)used; }
 int64_t fake_peak() { return (int64_t)peak; }
@@ -103,6 +104,7 @@ cudaError_t cudaFree(void* p) {
     }
     return cudaSuccess;
 }
+cudaError_t cudaMemGetInfo(size_t* f, size_t* t) { *f = limit - used; *t = limit; return cudaSuccess; }
 cudaError_t cudaMallocHost(void** p, size_t n) { *p = std::calloc(1, n ? n : 1); return cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { std::free(p); return cudaSuccess; }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { std::memcpy(d, s, n); return cudaSuccess; }

@@ -5,6 +5,7 @@ import ctypes
 import os
 import subprocess
 
+import numpy as np
 import pytest
 
 from mrlbm_2d_b200 import api
@@ -14,6 +15,9 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "mrlbm_2d_b200", "csrc")
 CUDA_INC = "/usr/local/cuda/include"
 STEP, PAIR, BATCH = 0, 1, 2
+
+fake_args = dict(fake_limit=[ctypes.c_int64], fake_pair_us=[ctypes.c_double], fake_step_us=[ctypes.c_int, ctypes.c_double],
+                 fake_fail=[ctypes.c_char_p, ctypes.c_int])
 
 pytestmark = pytest.mark.skipif(not os.path.isdir(CUDA_INC), reason="CUDA headers not installed")
 
@@ -27,6 +31,8 @@ def library(tmp_path_factory):
     L = api.load_library(out)
     for f in ("fake_used", "fake_peak", "fake_done", "fake_captures", "fake_dangling"):
         getattr(L, f).restype = ctypes.c_int64
+    for f, a in fake_args.items():
+        getattr(L, f).argtypes = a
     return L
 
 
@@ -48,8 +54,9 @@ def large():
     return cylinder_case(1400, 520, 40, 300.0, 260.5, 100.0, 0.05)
 
 
-def level_bytes(s):
-    return s.info.state_bytes
+def tuned_pairs(fake):
+    """Costs at which every autotuner takes pairs."""
+    fake.fake_pair_us(0.5)
 
 
 @pytest.mark.parametrize("prec", [64, 32])
@@ -64,3 +71,87 @@ def test_a_replay_that_cannot_be_made_is_launched_step_by_step(fake, prec, call)
     s.step(2600)                                             # not tried again for every run
     assert fake.fake_captures() == captures and fake.fake_done(STEP) == 5200
     s.close()
+
+
+LATER = {"macro": lambda s: s.step(5, macro=True), "field window": lambda s: s.field_stats_window(2, 100), "state": lambda s: s.get_state(),
+         "body force": lambda s: s.set_body_force(np.zeros((2, s.nx, s.ny))), "inlet profile": lambda s: s.set_inlet_profile(np.zeros(s.ny)),
+         "surface": lambda s: s.surface_enable(), "gradient": lambda s: s.adjoint_drag(20, 5, 6), "autotune": lambda s: s.autotune(4)}
+
+
+@pytest.mark.parametrize("what", sorted(LATER))
+def test_the_band_of_the_pairs_goes_back_when_memory_is_short(fake, monkeypatch, what):
+    """What fits beside a handle of single steps fits beside one that steps in pairs."""
+    cfg = large()
+    monkeypatch.setenv("MRLBM_PAIRS", "0")
+    s = api.Simulation(cfg)
+    single = fake.fake_used()
+    fake.fake_mark()
+    LATER[what](s)
+    need = fake.fake_peak()
+    s.close()
+    monkeypatch.delenv("MRLBM_PAIRS")
+    s = api.Simulation(cfg)
+    assert fake.fake_used() == single + s.info.state_bytes // 2          # pairs, with their third level
+    s.step(4)
+    assert fake.fake_done(PAIR) == 2
+    fake.fake_limit(max(need, fake.fake_used()))
+    LATER[what](s)
+    pairs = fake.fake_done(PAIR)
+    s.step(4)
+    assert s.status() == 0
+    if need > single + s.info.state_bytes // 2:
+        assert fake.fake_done(PAIR) == pairs                             # single steps since
+    s.close()
+
+
+def test_pairs_take_at_most_a_quarter_of_the_free_memory(fake):
+    cfg = large()
+    s = api.Simulation(cfg)
+    level, used = s.info.state_bytes // 2, fake.fake_used()
+    s.close()
+    for room, pairs in ((4 * level + 1000, 2), (4 * level - 1000, 0)):
+        fake.fake_reset()
+        fake.fake_limit(used - level + room)
+        s = api.Simulation(cfg)
+        s.step(4)
+        assert fake.fake_done(PAIR) == pairs
+        s.close()
+
+
+@pytest.mark.parametrize("forced", [False, True])
+def test_a_batch_is_created_in_the_memory_of_single_steps(fake, monkeypatch, forced):
+    cfgs = [large()] * 3
+    monkeypatch.setenv("MRLBM_PAIRS", "0")
+    fake.fake_mark()
+    b = api.Batch(cfgs, precision=64)
+    single = fake.fake_peak()
+    b.close()
+    if forced:
+        monkeypatch.setenv("MRLBM_PAIRS", "1")
+        fake.fake_limit(single)
+    else:
+        monkeypatch.delenv("MRLBM_PAIRS")
+    fake.fake_mark()
+    b = api.Batch(cfgs, precision=64)
+    assert fake.fake_peak() == single
+    fake.fake_limit(1 << 62)
+    b.step(10)
+    assert b.status() == 0
+    b.close()
+
+
+def test_a_batch_in_pairs_gives_its_bands_back(fake):
+    cfgs = [large()] * 3
+    b = api.Batch(cfgs, precision=64)
+    used = fake.fake_used()
+    tuned_pairs(fake)
+    b.autotune(8)
+    assert fake.fake_used() > used + 3 * (b.cases[0].info.state_bytes // 2)
+    b.step(16)
+    pairs = fake.fake_done(PAIR)
+    assert pairs > 0
+    fake.fake_limit(fake.fake_used() + 1000)
+    b.step(16, macro=True)                                               # three macroscopic buffers
+    b.step(16)
+    assert b.status() == 0
+    b.close()
