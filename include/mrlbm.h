@@ -249,7 +249,10 @@ int mrlbm_step_noalloc(mrlbm_handle* h, void* d_state, const double* d_f0, int32
  * Every shape computes the same bits.  The default is 1; MRLBM_TILE_CFG in
  * the environment overrides it at creation.  A shape that does not fit the handle's precision
  * makes the next mrlbm_step return MRLBM_EUNSUPPORTED.  mrlbm_step_noalloc runs shape 1 when a
- * TMA shape is selected (its counters live in the handle). */
+ * TMA shape is selected (its counters live in the handle).
+ * The shape is that of single steps.  Steps in pairs (mrlbm_step) have one of their own, and setting a shape leaves a
+ * handle's pairs as they are, so that a shape kept from an earlier mrlbm_autotune costs a new handle
+ * nothing; MRLBM_PAIRS=0 at creation makes every step one of the shape set here. */
 #define MRLBM_N_TILE_CONFIGS 31
 int mrlbm_set_tile_config(mrlbm_handle* h, int32_t cfg);
 int mrlbm_get_tile_config(const mrlbm_handle* h, int32_t* cfg);

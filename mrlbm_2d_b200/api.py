@@ -256,6 +256,7 @@ class Simulation:
 
     @property
     def tile_config(self):
+        """Bulk tile shape of single steps; steps taken in pairs (include/mrlbm.h) have one of their own."""
         c = ctypes.c_int32()
         self._check(self._L.mrlbm_get_tile_config(self._h, ctypes.byref(c)))
         return c.value
