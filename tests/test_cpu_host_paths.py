@@ -26,7 +26,7 @@ pytestmark = pytest.mark.skipif(not os.path.isdir(CUDA_INC), reason="CUDA header
 def library(tmp_path_factory):
     out = str(tmp_path_factory.mktemp("fake") / "libfake.so")
     srcs = [os.path.join(CSRC, f) for f in ("capi.cpp", "geometry.cpp", "statistics.cpp")]
-    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-I", CSRC, "-I", os.path.join(ROOT, "include"), "-I", CUDA_INC,
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I", CSRC, "-I", os.path.join(ROOT, "include"), "-I", CUDA_INC,
                     *srcs, os.path.join(ROOT, "tests", "fake_cuda.cpp"), "-o", out], check=True)
     L = api.load_library(out)
     for f in ("fake_used", "fake_peak", "fake_done", "fake_captures", "fake_dangling"):
