@@ -2081,6 +2081,9 @@ struct mrlbm_batch {
     // the autotuner's choice: per-case streams whose steps are taken in pairs (step_pair.cuh); every case then
     // has its band buffer
     bool pairs = false, pairs_fixed = false;   // fixed: by MRLBM_PAIRS at creation
+    // the schedule the autotuner left and whether its steps are paired: set again, it is the same schedule
+    int tuned_tile = -1, tuned_schedule = -1, tuned_steps = -1;
+    bool tuned_pairs = false;
 };
 
 namespace {
@@ -2574,7 +2577,13 @@ int mrlbm_batch_set_schedule(mrlbm_batch* b, int32_t tile_cfg, int32_t schedule,
     b->tile_cfg = tile_cfg;
     b->schedule = schedule;
     b->steps_per_launch = steps_per_launch;
-    if (!b->pairs_fixed) b->pairs = false;
+    if (!b->pairs_fixed) {
+        cudaSetDevice(b->device);
+        b->pairs = b->tuned_pairs && tile_cfg == b->tuned_tile && schedule == b->tuned_schedule && steps_per_launch == b->tuned_steps;
+        for (mrlbm_handle* h : b->h) b->pairs = b->pairs && enable_pairs(h, (int)b->h.size());
+        if (!b->pairs)
+            for (mrlbm_handle* h : b->h) disable_pairs(h);         // (freeing waits for the steps under way)
+    }
     return MRLBM_OK;
 }
 
@@ -2757,6 +2766,10 @@ int mrlbm_batch_autotune(mrlbm_batch* b, int32_t trial_steps, double* best_ms_pe
     b->tile_cfg = best_tile;
     b->schedule = best_sched;
     b->steps_per_launch = best_spl;
+    b->tuned_tile = best_tile;
+    b->tuned_schedule = best_sched;
+    b->tuned_steps = best_spl;
+    b->tuned_pairs = pairs_best;
     if (best_ms_per_step) *best_ms_per_step = best / steps;
     return MRLBM_OK;
 }

@@ -155,3 +155,21 @@ def test_a_batch_in_pairs_gives_its_bands_back(fake):
     b.step(16)
     assert b.status() == 0
     b.close()
+
+
+def test_a_schedule_set_by_hand_has_no_pairs_but_the_autotuners_has(fake):
+    b = api.Batch([large()] * 2, precision=64)
+    single = fake.fake_used()
+    tuned_pairs(fake)
+    tuned, _ = b.autotune(8)
+    paired = fake.fake_used()
+    b.set_schedule(3, api.BATCH_STREAMS, 8)
+    assert fake.fake_used() == paired - 2 * (b.cases[0].info.state_bytes // 2)    # the bands are back
+    pairs = fake.fake_done(PAIR)
+    b.step(16)
+    assert fake.fake_done(PAIR) == pairs
+    b.set_schedule(*tuned)
+    assert b.schedule == tuned and fake.fake_used() >= single + b.cases[0].info.state_bytes
+    b.step(16)
+    assert fake.fake_done(PAIR) == pairs + 16                                     # 8 pairs of each case
+    b.close()
