@@ -2730,16 +2730,18 @@ int mrlbm_batch_autotune(mrlbm_batch* b, int32_t trial_steps, double* best_ms_pe
         b->schedule = MRLBM_BATCH_STREAMS;
         b->steps_per_launch = steps;
         b->pairs = true;
-        // warm-up from either time level (an odd number of pairs changes it) and past a loaded state's first step
-        for (int w = 0; w < 3 && rc == MRLBM_OK; ++w) rc = batch_call(b, steps, 0);
-        if (rc == MRLBM_OK) {
+        // warm-up from either time level (an odd number of pairs changes it) and past a loaded state's first step;
+        // a trial that cannot be run (its graphs are larger than those of single steps) is one that is not faster
+        int prc = MRLBM_OK;
+        for (int w = 0; w < 3 && prc == MRLBM_OK; ++w) prc = batch_call(b, steps, 0);
+        if (prc == MRLBM_OK) {
             cudaEventRecord(e0, b->stream);
-            rc = batch_call(b, steps, 0);
+            prc = batch_call(b, steps, 0);
             cudaEventRecord(e1, b->stream);
-            if (rc == MRLBM_OK && cudaEventSynchronize(e1) != cudaSuccess) rc = MRLBM_ECUDA;
+            if (prc == MRLBM_OK && cudaEventSynchronize(e1) != cudaSuccess) rc = MRLBM_ECUDA;
             float ms = 0.f;
-            if (rc == MRLBM_OK) cudaEventElapsedTime(&ms, e0, e1);
-            if (rc == MRLBM_OK && ms < best) {
+            if (prc == MRLBM_OK && rc == MRLBM_OK) cudaEventElapsedTime(&ms, e0, e1);
+            if (prc == MRLBM_OK && rc == MRLBM_OK && b->pairs && ms < best) {
                 best = ms;
                 best_tile = streams_tile;
                 best_sched = MRLBM_BATCH_STREAMS;

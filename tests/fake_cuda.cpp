@@ -28,9 +28,9 @@ struct Graph { std::vector<Launch> nodes; };
 
 std::map<char*, size_t> live;
 size_t used = 0, peak = 0, limit = (size_t)1 << 60;
-std::map<std::string, int> failing;                 // call -> times it fails from now on
+std::map<std::string, std::pair<int, int>> failing; // call -> calls that still succeed, then times it fails
 double now = 0.0, step_us[N_ALL_CFGS], pair_us = 1.0, batch_us = 1e9;
-long long done[KINDS], dangling = 0, captures = 0;
+long long done[KINDS], dangling = 0, captures = 0, graphs = 0;
 Graph* capture = nullptr;
 cudaError_t last = cudaSuccess;
 
@@ -44,8 +44,9 @@ cudaError_t report(cudaError_t e) {
 }
 bool fails(const char* call) {
     auto it = failing.find(call);
-    if (it == failing.end() || it->second == 0) return false;
-    --it->second;
+    if (it == failing.end() || it->second.second == 0) return false;
+    if (it->second.first > 0) return --it->second.first, false;
+    --it->second.second;
     return true;
 }
 void run(const Launch& l) {
@@ -55,7 +56,7 @@ void run(const Launch& l) {
         if (!is_live(p)) ++dangling;
 }
 int launch(Kind kind, double us, std::vector<const void*> mem) {
-    if (fails("launch")) return -1;
+    if (fails("launch") || (kind == PAIR && fails("pair"))) return -1;
     Launch l{kind, us, std::move(mem)};
     if (capture) capture->nodes.push_back(l);
     else run(l);
@@ -73,9 +74,10 @@ void fake_reset() {
     pair_us = 1.0;
     batch_us = 1e9;
     std::fill(done, done + KINDS, 0);
-    dangling = captures = 0;
+    dangling = captures = graphs = 0;
 }
-void fake_fail(const char* call, int times) { failing[call] = times; }
+void fake_fail(const char* call, int times) { failing[call] = {0, times}; }
+void fake_fail_after(const char* call, int calls, int times) { failing[call] = {calls, times}; }
 void fake_mark() { peak = used; }
 void fake_limit(int64_t bytes) { limit = (size_t)bytes; }
 int64_t fake_used() { return (int64_t)used; }
@@ -84,6 +86,7 @@ void fake_step_us(int cfg, double us) { step_us[cfg] = us; }
 void fake_pair_us(double us) { pair_us = us; }
 int64_t fake_done(int kind) { return done[kind]; }
 int64_t fake_captures() { return captures; }
+int64_t fake_graphs() { return graphs; }
 int64_t fake_dangling() { return dangling; }
 
 // ---- the runtime
@@ -162,6 +165,7 @@ cudaError_t cudaGraphDestroy(cudaGraph_t g) { delete (Graph*)g; return cudaSucce
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t e) { delete (Graph*)e; return cudaSuccess; }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t e, cudaStream_t) {
     if (fails("cudaGraphLaunch")) return report(cudaErrorMemoryAllocation);
+    ++graphs;
     for (const Launch& l : ((Graph*)e)->nodes) run(l);
     return cudaSuccess;
 }

@@ -17,7 +17,7 @@ CUDA_INC = "/usr/local/cuda/include"
 STEP, PAIR, BATCH = 0, 1, 2
 
 fake_args = dict(fake_limit=[ctypes.c_int64], fake_pair_us=[ctypes.c_double], fake_step_us=[ctypes.c_int, ctypes.c_double],
-                 fake_fail=[ctypes.c_char_p, ctypes.c_int])
+                 fake_fail=[ctypes.c_char_p, ctypes.c_int], fake_fail_after=[ctypes.c_char_p, ctypes.c_int, ctypes.c_int])
 
 pytestmark = pytest.mark.skipif(not os.path.isdir(CUDA_INC), reason="CUDA headers not installed")
 
@@ -29,7 +29,7 @@ def library(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I", CSRC, "-I", os.path.join(ROOT, "include"), "-I", CUDA_INC,
                     *srcs, os.path.join(ROOT, "tests", "fake_cuda.cpp"), "-o", out], check=True)
     L = api.load_library(out)
-    for f in ("fake_used", "fake_peak", "fake_done", "fake_captures", "fake_dangling"):
+    for f in ("fake_used", "fake_peak", "fake_done", "fake_captures", "fake_graphs", "fake_dangling"):
         getattr(L, f).restype = ctypes.c_int64
     for f, a in fake_args.items():
         getattr(L, f).argtypes = a
@@ -172,4 +172,30 @@ def test_a_schedule_set_by_hand_has_no_pairs_but_the_autotuners_has(fake):
     assert b.schedule == tuned and fake.fake_used() >= single + b.cases[0].info.state_bytes
     b.step(16)
     assert fake.fake_done(PAIR) == pairs + 16                                     # 8 pairs of each case
+    b.close()
+
+
+@pytest.mark.parametrize("call", ["pair", "cudaGraphLaunch"])
+def test_batch_autotune_without_pairs_when_their_trial_fails(fake, call):
+    b = api.Batch([large()] * 2, precision=64)
+    tuned_pairs(fake)
+    used = fake.fake_used()
+    if call == "cudaGraphLaunch":                            # the paired trial's: after those of the shapes
+        fake.fake_reset()
+        tuned_pairs(fake)
+        b.autotune(8)
+        n = fake.fake_graphs()
+        b.close()
+        fake.fake_reset()
+        tuned_pairs(fake)
+        b = api.Batch([large()] * 2, precision=64)
+        used = fake.fake_used()
+        fake.fake_fail_after(call.encode(), n - 4, 1)
+    else:
+        fake.fake_fail(b"pair", 1)
+    b.autotune(8)
+    level = b.cases[0].info.state_bytes // 2
+    assert fake.fake_used() < used + level                   # no bands
+    b.step(16)
+    assert b.status() == 0
     b.close()
