@@ -1749,7 +1749,7 @@ int mrlbm_autotune(mrlbm_handle* h, int32_t trial_steps, int32_t* best_cfg, doub
     bool pairs_best = false;
     for (int c = 0; c < last && rc == MRLBM_OK; ++c) {
         const bool paired = c == N_ALL_CFGS;
-        h->pairs = h->pairs_fixed ? pairs0 : false;
+        h->pairs = false;                               // (also where pairs are fixed: the shape is single steps')
         if (paired) {
             if (best_t >= 1e30f || !enable_pairs(h)) break;
             h->tile_cfg = best;

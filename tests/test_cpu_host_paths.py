@@ -199,3 +199,14 @@ def test_batch_autotune_without_pairs_when_their_trial_fails(fake, call):
     b.step(16)
     assert b.status() == 0
     b.close()
+
+
+def test_autotune_times_shapes_by_single_steps_also_with_pairs_forced(fake, monkeypatch):
+    monkeypatch.setenv("MRLBM_PAIRS", "1")
+    s = api.Simulation(large())
+    fake.fake_step_us(7, 0.25)
+    assert s.autotune(6)[0] == 7
+    pairs = fake.fake_done(PAIR)
+    s.step(4)
+    assert fake.fake_done(PAIR) == pairs + 2                 # and the steps stay paired
+    s.close()
