@@ -261,8 +261,9 @@ int mrlbm_get_tile_config(const mrlbm_handle* h, int32_t* cfg);
  * warm-up step each), keep the fastest, and restore the populations, the iteration counter
  * and the force history, so a simulation is unaffected.  Trial steps record no surface
  * pressure; with a field-statistics window they accumulate like the run will (so the choice
- * fits it) into sums that are saved beforehand and put back.  With the fastest shape it then
- * times the steps in pairs (mrlbm_step) and keeps whichever is faster.  Returns the chosen shape
+ * fits it) into sums that are saved beforehand and put back.  On lattices above 400,000 nodes and at least 64
+ * nodes wide and high it then times the steps in pairs (mrlbm_step; an even number of steps, two at
+ * least) and keeps whichever is faster.  Returns the chosen shape
  * (of single steps) and the time per step in milliseconds. */
 int mrlbm_autotune(mrlbm_handle* h, int32_t trial_steps, int32_t* best_cfg, double* best_ms);
 

@@ -1739,51 +1739,57 @@ int mrlbm_autotune(mrlbm_handle* h, int32_t trial_steps, int32_t* best_cfg, doub
     int best = cfg0;
     float best_t = 1e30f;
     int rc = MRLBM_OK;
-    // every shape by single steps, then (index N_ALL_CFGS) the best of them with its steps in pairs, on
-    // lattices that are not so small that single steps were always the faster (pairs_pay)
     const bool pairs0 = h->pairs;
     const int64_t stepped0 = h->stepped;
-    h->no_replay = true;
-    const bool try_pairs = !h->pairs_fixed && std::min(h->L.nx, h->L.ny) >= 64 && (int64_t)h->L.nx * h->L.ny > REPLAY_MAX_NODES;
-    const int last = try_pairs ? N_ALL_CFGS + 1 : N_ALL_CFGS;
-    bool pairs_best = false;
-    for (int c = 0; c < last && rc == MRLBM_OK; ++c) {
-        const bool paired = c == N_ALL_CFGS;
-        h->pairs = false;                               // (also where pairs are fixed: the shape is single steps')
-        if (paired) {
-            if (best_t >= 1e30f || !enable_pairs(h)) break;
-            h->tile_cfg = best;
-        } else {
-            h->tile_cfg = c;
-        }
-        rc = mrlbm_step(h, paired ? 2 : 1, 0);          // warm-up (and instruction cache)
-        if (rc == MRLBM_EUNSUPPORTED) {                 // shape does not fit: nothing ran
-            rc = MRLBM_OK;
+    // Time per step of `steps` steps after `warm` untimed ones; every trial starts from the same state.
+    auto trial = [&](int warm, int steps, float& t) {
+        int trc = mrlbm_step(h, warm, 0);               // instruction cache, first launches
+        if (trc == MRLBM_EUNSUPPORTED) {                // shape does not fit: nothing ran
             h->iter = iter0;
-            continue;
+            return trc;
         }
-        if (rc != MRLBM_OK) break;
         cudaEventRecord(e0, h->stream);
-        rc = mrlbm_step(h, trial_steps, 0);
+        if (trc == MRLBM_OK) trc = mrlbm_step(h, steps, 0);
         cudaEventRecord(e1, h->stream);
-        if (rc != MRLBM_OK || cudaEventSynchronize(e1) != cudaSuccess) { rc = rc ? rc : MRLBM_ECUDA; break; }
         float ms = 0.f;
-        cudaEventElapsedTime(&ms, e0, e1);
-        if (ms < best_t) {
-            best_t = ms;
-            if (paired) pairs_best = true;
-            else best = c;
-        }
-        // restore before the next trial so every shape starts from the same state
+        if (trc == MRLBM_OK && (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess)) trc = MRLBM_ECUDA;
+        t = ms / steps;
         for (int b = 0; b < 2; ++b)
-            if (cudaMemcpyAsync(h->buf[b], save[b], bytes, cudaMemcpyDeviceToDevice, h->stream) != cudaSuccess)
-                rc = MRLBM_ECUDA;
+            if (cudaMemcpyAsync(h->buf[b], save[b], bytes, cudaMemcpyDeviceToDevice, h->stream) != cudaSuccess) rc = MRLBM_ECUDA;
         h->iter = iter0;
         h->cur = cur0;
         h->ring_n = ring0;
         h->ovr_live = ovr0;
         h->hist.resize(hist0);
         h->pend.on = false;                             // the trials' last record is discarded
+        return trc;
+    };
+    float t = 0.f;
+    h->no_replay = true;
+    h->pairs = false;                                   // (also where pairs are fixed: the shape is single steps')
+    for (int c = 0; c < N_ALL_CFGS && rc == MRLBM_OK; ++c) {
+        h->tile_cfg = c;
+        const int trc = trial(1, trial_steps, t);
+        if (trc == MRLBM_EUNSUPPORTED) continue;
+        if (trc != MRLBM_OK) rc = trc;
+        else if (t < best_t) {
+            best_t = t;
+            best = c;
+        }
+    }
+    // the best of them with its steps in pairs, on lattices that are not so small that single steps were always the
+    // faster (pairs_pay): an even number of steps, after enough for a loaded state's first step and a shape newly
+    // set, which are taken alone
+    bool pairs_best = false;
+    if (rc == MRLBM_OK && best_t < 1e30f && !h->pairs_fixed && std::min(h->L.nx, h->L.ny) >= 64 &&
+        (int64_t)h->L.nx * h->L.ny > REPLAY_MAX_NODES && enable_pairs(h)) {
+        h->tile_cfg = best;
+        if (trial(4, std::max(2, (trial_steps + 1) & ~1), t) != MRLBM_OK) {
+            cudaGetLastError();                         // not to be had; an error that stays fails the next call
+        } else if (h->paired() && t < best_t) {
+            best_t = t;
+            pairs_best = true;
+        }
     }
     h->surf_on = surf0;
     h->fstat_begin = fsb0;
@@ -1810,7 +1816,7 @@ int mrlbm_autotune(mrlbm_handle* h, int32_t trial_steps, int32_t* best_cfg, doub
     else if (pairs_best) h->pairs = true;
     else disable_pairs(h);
     if (best_cfg) *best_cfg = best;
-    if (best_ms) *best_ms = best_t / trial_steps;
+    if (best_ms) *best_ms = best_t;
     return MRLBM_OK;
 }
 

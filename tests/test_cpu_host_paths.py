@@ -210,3 +210,34 @@ def test_autotune_times_shapes_by_single_steps_also_with_pairs_forced(fake, monk
     s.step(4)
     assert fake.fake_done(PAIR) == pairs + 2                 # and the steps stay paired
     s.close()
+
+
+@pytest.mark.parametrize("trial_steps", [1, 2, 3, 20])
+@pytest.mark.parametrize("loaded", [False, True])
+def test_autotune_times_pairs_by_pairs(fake, trial_steps, loaded):
+    """Whole pairs, per step: not two single steps against each other, and no single step among them."""
+    s = api.Simulation(large())
+    if loaded:
+        s.load_state(s.get_state(), iter=1)
+    fake.fake_reset()
+    fake.fake_pair_us(1.9)                                   # single steps take 1 us each
+    _, ms = s.autotune(trial_steps)
+    assert ms == pytest.approx(0.95e-3, rel=1e-3)
+    fake.fake_reset()
+    fake.fake_pair_us(2.1)
+    _, ms = s.autotune(trial_steps)
+    assert ms == pytest.approx(1e-3, rel=1e-3)
+    s.close()
+
+
+def test_autotune_without_pairs_when_their_trial_fails(fake):
+    s = api.Simulation(large())
+    level = s.info.state_bytes // 2
+    used = fake.fake_used()
+    tuned_pairs(fake)
+    fake.fake_fail(b"pair", 1)
+    s.autotune(6)
+    assert fake.fake_used() < used and s.iter == 1           # single steps, without the third level
+    assert used - fake.fake_used() < 2 * level
+    s.step(6)
+    s.close()
