@@ -107,7 +107,7 @@ struct mrlbm_handle {
         uint64_t used = 0;
     } replay[N_REPLAYS];
     uint64_t replay_clock = 0;
-    int64_t stepped = 0;                      // steps taken by the handle, the autotuner's left out
+    int64_t asked[2] = {0, 0};                // steps asked for in calls that hold a run of REPLAY_STEPS[.]
     bool no_replay = false;                   // autotuner trials of single shapes
     bool replay_failed = false;               // a run could not be captured or launched: launched steps from then on
     int* d_call = nullptr;                    // call state of the replay (StepParams::call)
@@ -691,11 +691,19 @@ int launch_two(mrlbm_handle* h) {
 // a graph (with the same programmatic dependence) 1.0 us apart.  That bounds a step whose work is
 // shorter than its launches.  A run of REPLAY_STEPS steps is captured once per start level and
 // replayed; what differs from replay to replay (iteration, ring slot, the record still to be summed) comes
-// from the call state, copied ahead of it.  Calls of 400 steps and the read of their forces, us, launched
-// and replayed: 80 x 50 FP64 2100, 1620; 400 x 100 2100, 1690 (FP32 1520, 1395); 1003 x 251 2690, 2420
-// (FP32 2295, 2210); 1400 x 350 the same, its steps outlast their launches.
+// from the call state, copied ahead of it.  us per step of the default shape, launched and in runs of 16 and 64: FP64
+// 80 x 50 4.9, 3.85, 3.65; 400 x 100 4.9, 4.85, 4.6; 1003 x 251 6.6, 6.15, 5.95; 1260 x 315 8.3, 7.85, 7.65; FP32
+// 3.4, 3.45, 3.2; 3.7, 3.75, 3.45; 5.45, 5.3, 5.35; 5.7, 5.75, 5.5.  From 1400 x 350 on steps outlast their launches.
 constexpr int64_t REPLAY_MAX_NODES = 400000;
-constexpr int REPLAY_AFTER = 24;
+
+// Steps to be asked for, in calls that hold a run of n, before it is captured: about as many as save the
+// time of the capture (0.2 to 0.35 ms for 16 steps, 0.3 to 0.5 ms for 64), so that a handle used once loses
+// nothing and one used again little.  0: never, runs of 16 steps are no faster in FP32.
+int64_t replay_after(const mrlbm_handle* h, int n) {
+    if (n == REPLAY_STEPS[0]) return 1536;
+    if (h->precision == MRLBM_FP32) return 0;
+    return (int64_t)h->L.nx * h->L.ny <= 100000 ? 384 : 768;
+}
 
 // Length of the run to replay for the next `left` steps, or 0: launched steps.  Every step of the run must be
 // one whose launch differs from its captured form in the call state only.
@@ -704,12 +712,11 @@ int replay_length(const mrlbm_handle* h, int left) {
         (int64_t)h->L.nx * h->L.ny > REPLAY_MAX_NODES || h->halo_l || h->halo_r)
         return 0;
     const mrlbm_config& c = h->cfg;
-    for (int n : REPLAY_STEPS) {
-        const int a = h->iter + 1, z = h->iter + n;
+    for (int q = 0; q < 2; ++q) {
+        const int n = REPLAY_STEPS[q], a = h->iter + 1, z = h->iter + n;
         if (left < n || h->ring_n + n > RING_CAP) continue;
-        // capturing costs 0.3 ms for 16 and 0.7 ms for 64 steps, a replayed step saves 0.5 to 1.2 us: not
-        // before the handle has been asked for the steps that pay for it
-        if (h->stepped + left < REPLAY_AFTER * n) continue;
+        const int64_t after = replay_after(h, n);
+        if (after == 0 || h->asked[q] < after) continue;
         const bool fields = h->d_fstat && std::max(a, h->fstat_begin) <= std::min(z, h->fstat_end);
         if (fields && !(h->fstat_begin <= a && z <= h->fstat_end)) continue;       // all of the run or none of it
         // a plot step's solid velocities follow the call state in the tile shapes only
@@ -1531,11 +1538,12 @@ int mrlbm_step(mrlbm_handle* h, int32_t nsteps, int32_t flags) {
     CK(cudaSetDevice(h->device));
     if ((flags & MRLBM_STEP_MACRO) && !h->d_macro)
         CK(device_alloc(h, (void**)&h->d_macro, (size_t)6 * h->L.nx * h->L.ny * sizeof(double)));
+    const int runs = nsteps - ((flags & MRLBM_STEP_MACRO) ? 1 : 0);   // a step with macroscopic output is taken alone
+    for (int q = 0; q < 2; ++q)
+        if (runs >= REPLAY_STEPS[q] && !h->no_replay) h->asked[q] += runs;
     for (int s = 0; s < nsteps;) {
         int rc;
-        // a step with macroscopic output is taken alone
-        const int s0 = s;
-        const int run = replay_length(h, nsteps - s - ((flags & MRLBM_STEP_MACRO) ? 1 : 0));
+        const int run = replay_length(h, runs - s);
         if (run > 0 && step_replay(h, run)) {
             s += run;
         } else if (nsteps - s >= ((flags & MRLBM_STEP_MACRO) ? 3 : 2) && pair_ok(h)) {
@@ -1552,7 +1560,6 @@ int mrlbm_step(mrlbm_handle* h, int32_t nsteps, int32_t flags) {
             }
             ++s;
         }
-        h->stepped += s - s0;
         if (h->ring_n == RING_CAP) {
             rc = drain_ring(h);
             if (rc != MRLBM_OK) return rc;
@@ -1740,7 +1747,6 @@ int mrlbm_autotune(mrlbm_handle* h, int32_t trial_steps, int32_t* best_cfg, doub
     float best_t = 1e30f;
     int rc = MRLBM_OK;
     const bool pairs0 = h->pairs;
-    const int64_t stepped0 = h->stepped;
     // Time per step of `steps` steps after `warm` untimed ones; every trial starts from the same state.
     auto trial = [&](int warm, int steps, float& t) {
         int trc = mrlbm_step(h, warm, 0);               // instruction cache, first launches
@@ -1805,7 +1811,6 @@ int mrlbm_autotune(mrlbm_handle* h, int32_t trial_steps, int32_t* best_cfg, doub
     cudaStreamSynchronize(h->stream);
     cleanup();
     h->no_replay = false;
-    h->stepped = stepped0;
     if (rc != MRLBM_OK) {
         h->tile_cfg = cfg0;
         h->pairs = pairs0;

@@ -241,3 +241,19 @@ def test_autotune_without_pairs_when_their_trial_fails(fake):
     assert used - fake.fake_used() < 2 * level
     s.step(6)
     s.close()
+
+
+@pytest.mark.parametrize("prec,nodes,calls,captures", [
+    (64, "small", [383], 0), (64, "small", [384], 1), (64, "small", [200, 200], 1), (64, "small", [1536], 1),
+    (64, "mid", [767], 0), (64, "mid", [768], 1),
+    (32, "small", [800], 0), (32, "small", [1535], 0), (32, "small", [1536], 1), (32, "mid", [800], 0),
+    # steps of calls too short for a run do not count towards it
+    (64, "small", [1] * 5000 + [64], 0), (32, "small", [40] * 50 + [64], 0), (64, "small", [15] * 100 + [300], 0)])
+def test_runs_are_captured_once_calls_that_hold_them_pay_for_it(fake, prec, nodes, calls, captures):
+    cfg = small() if nodes == "small" else cylinder_case(400, 260, 20, 100.0, 130.5, 100.0, 0.05)
+    s = api.Simulation(cfg, precision=prec)
+    for n in calls:
+        s.step(n)
+    assert (fake.fake_captures() > 0) == (captures > 0)
+    assert fake.fake_done(STEP) == sum(calls)
+    s.close()
