@@ -29,7 +29,7 @@ struct Graph { std::vector<Launch> nodes; };
 std::map<char*, size_t> live;
 size_t used = 0, peak = 0, limit = (size_t)1 << 60;
 std::map<std::string, std::pair<int, int>> failing; // call -> calls that still succeed, then times it fails
-double now = 0.0, step_us[N_ALL_CFGS], pair_us = 1.0, batch_us = 1e9;
+double now = 0.0, step_us[N_ALL_CFGS], pair_us = 1.0, batch_us = 1e9, graph_factor = 1.0;
 long long done[KINDS], dangling = 0, captures = 0, graphs = 0;
 Graph* capture = nullptr;
 cudaError_t last = cudaSuccess;
@@ -49,9 +49,9 @@ bool fails(const char* call) {
     --it->second.second;
     return true;
 }
-void run(const Launch& l) {
+void run(const Launch& l, double factor = 1.0) {
     ++done[l.kind];
-    now += l.us;
+    now += factor * l.us;
     for (const void* p : l.mem)
         if (!is_live(p)) ++dangling;
 }
@@ -73,6 +73,7 @@ void fake_reset() {
     for (double& u : step_us) u = 1.0;
     pair_us = 1.0;
     batch_us = 1e9;
+    graph_factor = 1.0;
     std::fill(done, done + KINDS, 0);
     dangling = captures = graphs = 0;
 }
@@ -84,6 +85,7 @@ int64_t fake_used() { return (int64_t)used; }
 int64_t fake_peak() { return (int64_t)peak; }
 void fake_step_us(int cfg, double us) { step_us[cfg] = us; }
 void fake_pair_us(double us) { pair_us = us; }
+void fake_graph_factor(double f) { graph_factor = f; }
 int64_t fake_done(int kind) { return done[kind]; }
 int64_t fake_captures() { return captures; }
 int64_t fake_graphs() { return graphs; }
@@ -166,7 +168,7 @@ cudaError_t cudaGraphExecDestroy(cudaGraphExec_t e) { delete (Graph*)e; return c
 cudaError_t cudaGraphLaunch(cudaGraphExec_t e, cudaStream_t) {
     if (fails("cudaGraphLaunch")) return report(cudaErrorMemoryAllocation);
     ++graphs;
-    for (const Launch& l : ((Graph*)e)->nodes) run(l);
+    for (const Launch& l : ((Graph*)e)->nodes) run(l, graph_factor);
     return cudaSuccess;
 }
 static CUresult encode_tiled(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,

@@ -16,7 +16,7 @@ CSRC = os.path.join(ROOT, "mrlbm_2d_b200", "csrc")
 CUDA_INC = "/usr/local/cuda/include"
 STEP, PAIR, BATCH = 0, 1, 2
 
-fake_args = dict(fake_limit=[ctypes.c_int64], fake_pair_us=[ctypes.c_double], fake_step_us=[ctypes.c_int, ctypes.c_double],
+fake_args = dict(fake_limit=[ctypes.c_int64], fake_pair_us=[ctypes.c_double], fake_graph_factor=[ctypes.c_double], fake_step_us=[ctypes.c_int, ctypes.c_double],
                  fake_fail=[ctypes.c_char_p, ctypes.c_int], fake_fail_after=[ctypes.c_char_p, ctypes.c_int, ctypes.c_int])
 
 pytestmark = pytest.mark.skipif(not os.path.isdir(CUDA_INC), reason="CUDA headers not installed")
@@ -227,6 +227,35 @@ def test_autotune_times_pairs_by_pairs(fake, trial_steps, loaded):
     fake.fake_pair_us(2.1)
     _, ms = s.autotune(trial_steps)
     assert ms == pytest.approx(1e-3, rel=1e-3)
+    s.close()
+
+
+@pytest.mark.parametrize("prec", [64, 32])
+@pytest.mark.parametrize("loaded", [False, True])
+@pytest.mark.parametrize("replayed,chosen", [(0.8, 4), (0.95, 10)])
+def test_autotune_times_a_tma_shape_against_replayed_runs(fake, prec, loaded, replayed, chosen):
+    """Every shape but the TMA ones is replayed on small lattices; the launched steps of all are timed."""
+    s = api.Simulation(small(), precision=prec)
+    if loaded:
+        s.load_state(s.get_state(), iter=1)
+    fake.fake_step_us(4, 0.99)
+    fake.fake_step_us(10, 0.9)
+    fake.fake_graph_factor(replayed)
+    cfg, ms = s.autotune(6)
+    assert cfg == chosen and ms == pytest.approx(min(0.9, 0.99 * replayed) * 1e-3, rel=1e-3)
+    s.step(300)                                              # the trial's run does not count as asked for
+    assert fake.fake_captures() == 1 and s.iter == 301
+    s.close()
+
+
+def test_autotune_keeps_a_tma_shape_where_runs_are_not_replayed(fake):
+    cfg = cylinder_case(1003, 403, 60, 250.0, 201.5, 120.0, 0.05)
+    s = api.Simulation(cfg, precision=32)
+    fake.fake_step_us(10, 0.9)
+    fake.fake_pair_us(1e3)
+    fake.fake_graph_factor(0.1)
+    assert s.autotune(6)[0] == 10
+    assert fake.fake_captures() == 0
     s.close()
 
 
